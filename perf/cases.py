@@ -184,3 +184,73 @@ def tolerance(case):
     bf16 0.0030 relative (2-norm) and 0.022 of one value; fp16, whose gate is evaluated in fp16 pairs, 0.00098 and
     0.0145."""
     return {"rel": 0.012, "max": 0.09} if case["dtype"] == "bf16" else {"rel": 0.004, "max": 0.06}
+
+
+def _splitmix(x):
+    """splitmix64 on int64 tensors (the arithmetic wraps; the shifts are logical)."""
+    x = x + (0x9E3779B97F4A7C15 - (1 << 64))
+    x = (x ^ ((x >> 30) & ((1 << 34) - 1))) * (0xBF58476D1CE4E5B9 - (1 << 64))
+    x = (x ^ ((x >> 27) & ((1 << 37) - 1))) * (0x94D049BB133111EB - (1 << 64))
+    return x ^ ((x >> 31) & ((1 << 33) - 1))
+
+
+def _kept(seed, M, K, p, dev):
+    """The dropout mask of one group, over 1 - p: element (m, k) stays if its 24-bit hash is at least p."""
+    h = _splitmix(_splitmix(seed + 0xDEADBEEF) ^ _splitmix(torch.arange(M * K, device=dev))) >> 40 & ((1 << 24) - 1)
+    return ((h.float() / (1 << 24)) >= p).double().view(M, K) / (1.0 - p)
+
+
+def _shuffled(masks, K):
+    """Where each of a group's features is taken from: pairs of features change places by two rounds of swaps in each
+    chunk of 64, one mask bit a pair of segments."""
+    G, chunks, rounds = masks.shape
+    seg = torch.arange(32, device=masks.device).expand(G, chunks, 32).clone()
+    for r, delta in enumerate((8, 16)):
+        low = torch.tensor([i for i in range(32) if not i & delta], device=masks.device)
+        swap = (masks[:, :, r, None] >> torch.arange(16, device=masks.device) & 1).bool()
+        a, b = seg[..., low].clone(), seg[..., low + delta].clone()
+        seg[..., low], seg[..., low + delta] = torch.where(swap, b, a), torch.where(swap, a, b)
+    at = torch.arange(0, K, 64, device=masks.device)[None, :, None, None] + 2 * seg[..., None]
+    return (at + torch.arange(2, device=masks.device)).reshape(G, K)
+
+
+def exact(case, seed):
+    """The formulas in float64, group by group, with autograd for the gradients."""
+    state, c = prepare(case, seed), case
+    M, K, N, gs, rs, G = c["M"], c["K"], c["N"], c["gs"], c["rs"], c["N"] // c["gs"]
+    back, layer = c["call"] in ("step", "train"), state.get("layer")
+    B, R, ib = (state["B"], state["R"], state["fwd"].get("internal_bias")) if layer is None else (
+        layer.weight, layer.reconn, layer._internal_bias)
+    A, dC = state["A"].detach().double().requires_grad_(back), state["dC"]
+    P = [None if t is None else t.detach().double().requires_grad_(back) for t in (B, R, ib)]
+    perm = _shuffled(layer._shuffle_masks, K) if c["shuffle"] else None
+    y, grads, dA = torch.empty(M, N, dtype=torch.float64, device=A.device), [[], [], []], torch.zeros_like(A)
+    for g in range(G):
+        b, r, i = (None if t is None else t.view(G, -1, K)[g] for t in P)
+        r = r.reshape(rs, K // rs, rs).transpose(0, 1)
+        if layer is not None and c["act"] == "plain":   # the module holds the Cayley parameter
+            s, eye = r - r.mT, torch.eye(rs, dtype=torch.float64, device=A.device)
+            r = torch.linalg.solve(eye - s, eye + s)
+        a = A if perm is None else A[:, perm[g]]
+        s = torch.einsum("mbj,bij->mbi", a.view(M, K // rs, rs), r).reshape(M, K)
+        s = s if i is None else s + i
+        h = {"plain": lambda: s, "silu": lambda: a * s * torch.sigmoid(s), "sigmoid": lambda: 2 * a * torch.sigmoid(s)}[c["act"]]()
+        if c["p"] > 0:
+            h = h * _kept(state["fwd"]["dropout_seeds"][g], M, K, c["p"], A.device)
+        out = h @ b.mT
+        y[:, g * gs:(g + 1) * gs] = out.detach()
+        if back:
+            got = torch.autograd.grad(out, [A] + [t for t in P if t is not None], dC[:, g * gs:(g + 1) * gs].double())
+            dA += got[0]
+            for k, t in enumerate(got[1:]):   # a view's gradient is zero outside its group
+                grads[k].append(t.view(G, -1, K)[g].clone())
+    if layer is not None and layer.bias is not None:
+        y += layer.bias.detach().double()
+    if not back:
+        return y
+    dB, dR, d_ib = (torch.cat(t) if t else None for t in grads)
+    if layer is None:
+        return y, dA, dR, None if c["act"] == "plain" else dB, d_ib
+    gain = {"plain": 1.0, "silu": 1.437, "sigmoid": 1.15}[c["act"]]   # the layer divides its gradients by this, its bias's not
+    out = [y, dA / gain] + ([] if c["act"] == "plain" else [dB / gain]) + [dR / gain]
+    return out + ([dC.double().sum(0)] if c["bias"] else []) + ([] if d_ib is None else [d_ib / gain])
