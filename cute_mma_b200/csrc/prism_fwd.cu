@@ -19,7 +19,9 @@
 //   warps 4-19  gate warps, two groups of eight that take alternate chunks, 16 rows per warp: S from
 //               TMEM (tcgen05.ld delivers the accumulator-fragment layout), A by ldmatrix (same layout),
 //               H = A*silu(S) (or H = S) on registers, H back to TMEM over the first half of the S slot
-//   warps 20-23 epilogue: tcgen05.ld C, + bias, cast, swizzled staging tile, TMA store.
+//   warps 20-23 epilogue: tcgen05.ld C, + bias, cast, swizzled staging tile, TMA store.  The accumulator is
+//               single-buffered (TMEM is full), so the next tile's dense product waits for it to be read: it is
+//               released before its last columns are packed and stored.
 // Both products run on tcgen05: mma.sync shares the tensor cores with tcgen05.mma and is starved
 // while tcgen05.mma bursts run, so a rotation on mma.sync serialises the gate warps with the dense
 // product.  The issuing thread runs alone on its instruction stream (a barrier test costs it ~65
@@ -43,7 +45,8 @@ constexpr int kSlots = 4;             // TMEM slots of 64 columns: S (fp32), the
 constexpr int kSlotCol0 = 256;        // accumulator: TMEM columns [0, 256); slots: [256, 512)
 constexpr int kMaxStages = 8;
 constexpr int kATileBytes = 128 * 128;   // [128 rows x 64 elems] 16-bit
-constexpr int kEpiStageBytes = 32 * 128; // per epilogue warp: [32 rows x 64 elems]
+constexpr int kEpiStageBytes = 32 * 128; // per epilogue warp: [32 rows x 64 elems] ...
+constexpr int kEpiBiasBytes = 256 * 2;   // ... and the tile's bias
 }  // namespace fwd
 
 struct FwdParams {
@@ -86,6 +89,39 @@ __device__ __forceinline__ void tile_coords(const FwdParams& p, int t, int& mt, 
   mt = m0 + (rem - nt * pm);
 }
 
+// Epilogue of 32 columns: TMEM -> registers, + bias (from the warp's copy in shared memory), cast, half `hh` of the
+// swizzled [32 x 64] staging tile.  `release`: the accumulator's last columns are in registers, the next tile may
+// overwrite it.
+template <int DT, bool BIAS>
+__device__ __forceinline__ void epilogue_cols32(uint32_t tacc, uint8_t* stage, int lane, int hh, const uint4* bias,
+                                                uint32_t release) {
+  uint32_t v[32];
+  tmem_ld_x32(tacc, v);
+  tmem_ld_wait();
+  if (release != 0) {
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(release);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t ow[4];
+    const uint4 b4 = BIAS ? bias[j] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float x0 = __uint_as_float(v[j * 8 + e * 2]);
+      float x1 = __uint_as_float(v[j * 8 + e * 2 + 1]);
+      if (BIAS) {
+        const float2 b2 = Elem<DT>::unpack(e == 0 ? b4.x : e == 1 ? b4.y : e == 2 ? b4.z : b4.w);
+        x0 += b2.x;
+        x1 += b2.y;
+      }
+      ow[e] = Elem<DT>::pack(x0, x1);
+    }
+    *reinterpret_cast<uint4*>(stage + sw128_offset(lane, hh * 4 + j)) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+  }
+}
+
 // EXTRA: 0 the plain gate warps; 1 internal bias (a null bias is allowed); 2 hash dropout (+ optional bias)
 template <int DT, int GATE, int E, int EXTRA>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(fwd::kThreads, 1)
@@ -103,7 +139,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int b_bytes = p.BN * 64;   // BN/2 rows of 128 bytes
   uint8_t* smemSt = smem;
   uint8_t* smemEpi = smemSt + p.ns * p.stage_bytes;
-  FwdBarriers* bars = reinterpret_cast<FwdBarriers*>(smemEpi + kNumEpiWarps * kEpiStageBytes);
+  FwdBarriers* bars = reinterpret_cast<FwdBarriers*>(smemEpi + kNumEpiWarps * (kEpiStageBytes + kEpiBiasBytes));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -322,12 +358,23 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const uint32_t lane_base = uint32_t(q * 32) << 16;
     uint8_t* stage = smemEpi + (warp - kEpiWarp0) * kEpiStageBytes;
     const uint16_t* bias = reinterpret_cast<const uint16_t*>(p.bias);
+    uint4* bias_sm = reinterpret_cast<uint4*>(smemEpi + kNumEpiWarps * kEpiStageBytes) + (warp - kEpiWarp0) * 32;
+    const uint32_t acc_empty = mapa_shared(smem_u32(&bars->acc_empty), 0);
     uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = cid; t < p.n_tiles && ok; t += n_clusters, acc_phase ^= 1u) {
       int mp, nt;
       tile_coords(p, t, mp, nt);
       const int mt = mp * 2 + (int)rank;   // this CTA's 128-row block
+      if (p.tma_store && bias != nullptr && lane * 8 < p.BN) {
+        // This tile's bias, eight columns per lane, while the accumulator is still being formed: loaded pair by pair
+        // inside the epilogue it was the longer part of a short tile (16384 x 768 -> 3072: 124 us with a bias, 86 without).
+        const uint16_t* bp = bias + nt * p.BN + lane * 8;
+        const uint32_t* bw = reinterpret_cast<const uint32_t*>(bp);
+        bias_sm[lane] = reinterpret_cast<uintptr_t>(bias) % 16 == 0 ? __ldg(reinterpret_cast<const uint4*>(bp))
+                                                                    : make_uint4(__ldg(bw), __ldg(bw + 1), __ldg(bw + 2), __ldg(bw + 3));
+      }
+      __syncwarp();
       if (!mbar_wait(&bars->acc_full, acc_phase)) { ok = false; break; }
       const uint32_t tacc = tmem_base + lane_base;
       tc_fence_after_sync();
@@ -340,26 +387,9 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           __syncwarp();
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            uint32_t v[32];
-            tmem_ld_x32(tacc + c0 + hh * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint32_t ow[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                float x0 = __uint_as_float(v[j * 8 + e * 2]);
-                float x1 = __uint_as_float(v[j * 8 + e * 2 + 1]);
-                if (bias != nullptr) {
-                  const uint32_t bw = *reinterpret_cast<const uint32_t*>(bias + n0 + c0 + hh * 32 + j * 8 + e * 2);
-                  const float2 b2 = Elem<DT>::unpack(bw);
-                  x0 += b2.x;
-                  x1 += b2.y;
-                }
-                ow[e] = Elem<DT>::pack(x0, x1);
-              }
-              *reinterpret_cast<uint4*>(stage + sw128_offset(lane, hh * 4 + j)) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-            }
+            const uint32_t rel = (hh == 1 && c0 + 64 >= p.BN) ? acc_empty : 0u;
+            if (bias != nullptr) epilogue_cols32<DT, true>(tacc + c0 + hh * 32, stage, lane, hh, bias_sm + c0 / 8 + hh * 4, rel);
+            else epilogue_cols32<DT, false>(tacc + c0 + hh * 32, stage, lane, hh, nullptr, rel);
           }
           fence_proxy_async_smem();
           __syncwarp();
@@ -395,9 +425,11 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty), 0));
+      if (!p.tma_store) {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc_empty);
+      }
     }
     if (lane == 0) tma_store_wait_all<0>();   // outstanding stores read shared memory
     if (!ok && lane == 0) { atomicExch(p.err, PRISM_ERR_DEVICE_WAIT); }
@@ -432,7 +464,7 @@ int launch_fwd(const FwdArgs& a) {
   p.drop_seeds = a.drop_seeds; p.drop_p = a.drop_p; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "forward: dropout needs reconn_sz 8 or 16");
 
-  const int budget = 227 * 1024 - 1024 - (int)sizeof(FwdBarriers) - 256 - fwd::kNumEpiWarps * fwd::kEpiStageBytes;
+  const int budget = 227 * 1024 - 1024 - (int)sizeof(FwdBarriers) - 256 - fwd::kNumEpiWarps * (fwd::kEpiStageBytes + fwd::kEpiBiasBytes);
   p.stage_bytes = fwd::kATileBytes + p.r_tile_bytes + a.BN * 64;   // A tile, halves of the R and B tiles
   int ns = a.sa > 0 ? a.sa : fwd::kMaxStages;
   if (ns > fwd::kMaxStages) ns = fwd::kMaxStages;
@@ -440,7 +472,7 @@ int launch_fwd(const FwdArgs& a) {
   if (ns < fwd::kSlots || ns * p.stage_bytes > budget)   // a stage per TMEM slot at least (see the rotation issuer)
     return fail(PRISM_ERR_UNSUPPORTED, "forward tile does not fit shared memory (BN=%d E=%d)", a.BN, a.E);
   p.ns = ns;
-  const int smem_bytes = ns * p.stage_bytes + fwd::kNumEpiWarps * fwd::kEpiStageBytes +
+  const int smem_bytes = ns * p.stage_bytes + fwd::kNumEpiWarps * (fwd::kEpiStageBytes + fwd::kEpiBiasBytes) +
                          (int)sizeof(FwdBarriers) + 1024;
 
   CUtensorMap tmA, tmR, tmB, tmC;

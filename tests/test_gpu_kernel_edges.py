@@ -1,0 +1,28 @@
+"""Edges of the kernels' tiles, plans and copies, against the oracle in fp32 on the same 16-bit-rounded inputs.
+
+TOL is the reference's bar for 16-bit outputs (tests/test_correctness.py:24-31), as in test_gpu_parity.py."""
+import pytest
+import torch
+
+import cute_mma_b200 as cp
+from oracle import prism_oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-2
+DEV = "cuda"
+
+
+def _inputs(M, K, N, gs, rs, dt, seed=0):
+    return [t.to(dt).to(DEV).contiguous() for t in O.make_inputs(M, K, N, gs, rs, seed=seed, b_std=K ** -0.5)]
+
+
+@pytest.mark.parametrize("offset", [0, 2])          # 16-byte and 4-byte aligned bias
+@pytest.mark.parametrize("gs,N", [(256, 2560), (64, 192), (96, 288)])
+def test_bias_in_the_forward_epilogue(gs, N, offset):
+    """Several tiles per CTA pair (a bias of its own each), narrow tiles, and the plain-store epilogue (gs 96)."""
+    M, K, rs, dt = 4100, 128, 16, torch.bfloat16
+    A, B, R, _ = _inputs(M, K, N, gs, rs, dt, 3)
+    bias = torch.randn(N + 8, device=DEV).to(dt)[offset:offset + N]
+    C, _ = cp.forward(A, B, R, gs, rs, activation="silu_gate", bias=bias)
+    cp.check_device_status()
+    assert O.rel_err(C.float(), O.prism_forward(A.float(), B.float(), R.float(), gs, rs, "silu_gate", bias=bias.float())) < TOL
