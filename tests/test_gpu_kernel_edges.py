@@ -26,3 +26,18 @@ def test_bias_in_the_forward_epilogue(gs, N, offset):
     C, _ = cp.forward(A, B, R, gs, rs, activation="silu_gate", bias=bias)
     cp.check_device_status()
     assert O.rel_err(C.float(), O.prism_forward(A.float(), B.float(), R.float(), gs, rs, "silu_gate", bias=bias.float())) < TOL
+
+
+@pytest.mark.parametrize("gs", [48, 96, 160, 192, 224, 288])
+@pytest.mark.parametrize("rs", [8, 64])
+def test_tile_width_of_odd_groups(gs, rs):
+    """Groups whose widest tile is no power of two: forward (TMA and plain stores), dB and dA+dR."""
+    M, K, N, dt, act = 300, 192, 2 * gs, torch.float16, "silu_gate"
+    A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 5)
+    C, _ = cp.forward(A, B, R, gs, rs, activation=act)
+    dA, dR, dB, _ = cp.backward(dC, A, B, R, gs, rs, activation=act)
+    cp.check_device_status()
+    f = [t.float() for t in (A, B, R)]
+    rA, rR, rB = O.prism_backward(dC.float(), *f, gs, rs, act)
+    for got, ref in ((C, O.prism_forward(*f, gs, rs, act)), (dA, rA), (dR, rR), (dB, rB)):
+        assert O.rel_err(got.float(), ref) < TOL
