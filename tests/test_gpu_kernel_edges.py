@@ -41,3 +41,16 @@ def test_tile_width_of_odd_groups(gs, rs):
     rA, rR, rB = O.prism_backward(dC.float(), *f, gs, rs, act)
     for got, ref in ((C, O.prism_forward(*f, gs, rs, act)), (dA, rA), (dR, rR), (dB, rB)):
         assert O.rel_err(got.float(), ref) < TOL
+
+
+@pytest.mark.parametrize("K,rs", [(72, 8), (2056, 8), (2080, 16)])   # one warp; past one pass of a block; odd blocks of 8
+def test_widened_and_halved_rotation(K, rs):
+    M, N, gs, dt, act = 130, 256, 128, torch.bfloat16, "silu_gate"
+    A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 7)
+    C, _ = cp.forward(A, B, R, gs, rs, activation=act)
+    dA, dR, dB, _ = cp.backward(dC, A, B, R, gs, rs, activation=act)
+    cp.check_device_status()
+    f = [t.float() for t in (A, B, R)]
+    rA, rR, rB = O.prism_backward(dC.float(), *f, gs, rs, act)
+    for got, ref in ((C, O.prism_forward(*f, gs, rs, act)), (dA, rA), (dR, rR), (dB, rB)):
+        assert O.rel_err(got.float(), ref) < TOL
