@@ -315,14 +315,24 @@ __global__ void db_reduce_kernel(const float* __restrict__ partial, void* __rest
     *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dB_out) + (long long)n * lddb + k) = Elem<DT>::pack(acc.x, acc.y);
 }
 
+// Token-range splits of every tile: the count with the least estimated time, in units of one token block of a CTA pair
+// (about 1.1 us at BN = 256): waves of pairs x (blocks per pair + 3 for a pair's start and epilogue), and, when split, the
+// second launch with the fp32 partial sums written and read once (8 bytes each, about 6 TB/s).  Splitting pays when the
+// tiles leave most SM pairs idle; a count that only turns one wave into three shorter ones does not (4096 tokens, 1024 ->
+// 4096: 64 tiles on 74 pairs; three splits and their sum 69.5 us, none 41.2).
 static int db_default_splits(int M, int N, int K, int BN, int num_sms) {
-  const int base = 2 * ((K + 255) / 256) * (N / BN);
+  const long long tiles = (long long)((K + 255) / 256) * (N / BN);
   const int tokblocks = (M + 127) / 128;
-  if (base >= 2 * num_sms) return 1;
-  int s = (2 * num_sms + base - 1) / base;
-  if (s > tokblocks) s = tokblocks;
-  if (s > 16) s = 16;
-  return s < 1 ? 1 : s;
+  const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
+  int best = 1;
+  double best_cost = 0;
+  for (int s = 1; s <= 16 && s <= tokblocks; ++s) {
+    const long long waves = (tiles * s + pairs - 1) / pairs;
+    double cost = (double)waves * ((tokblocks + s - 1) / s + 3);
+    if (s > 1) cost += 4.0 + (double)s * N * K * 8.0 / 6.6e6;
+    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+  }
+  return best;
 }
 
 // Launch plan.  cfg = {BN, splits} or null: splits > 0 splits the token range of every tile, splits < 0

@@ -54,3 +54,17 @@ def test_widened_and_halved_rotation(K, rs):
     rA, rR, rB = O.prism_backward(dC.float(), *f, gs, rs, act)
     for got, ref in ((C, O.prism_forward(*f, gs, rs, act)), (dA, rA), (dR, rR), (dB, rB)):
         assert O.rel_err(got.float(), ref) < TOL
+
+
+@pytest.mark.parametrize("M,K,N,gs", [(128, 256, 256, 256),       # one token block: never split
+                                      (129, 264, 512, 256),       # two blocks, features past the first pair
+                                      (2200, 256, 256, 128),      # few tiles: split as often as it pays
+                                      (4096, 1024, 4096, 256)])   # 64 tiles: one wave, not split
+@pytest.mark.parametrize("out", [None, torch.float32])
+def test_split_plan_of_db(M, K, N, gs, out):
+    rs, dt, act = 16, torch.bfloat16, "sigmoid_gate"
+    A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 9)
+    dB = cp.backward(dC, A, B, R, gs, rs, activation=act, dB_dtype=out)[2]
+    cp.check_device_status()
+    ref = O.prism_backward(dC.float(), A.float(), B.float(), R.float(), gs, rs, act)[2]
+    assert dB.dtype == (out or dt) and O.rel_err(dB.float(), ref) < TOL
