@@ -344,6 +344,45 @@ def cayley_backward(M, dR, reconn_sz: int):
     return dM
 
 
+def _segment_aligned(X):
+    """X, or a copy of it where its first element does not start a pair of elements in memory."""
+    X = X.contiguous()
+    return X if X.data_ptr() % (2 * X.element_size()) == 0 else X.clone()
+
+
+def shuffle_cols(X, seg):
+    """Columns of a per-group matrix (G * rows, K) in another order, chunk by chunk: segment i (two features) of the
+    result is segment ``seg[g, chunk, i]`` of X, through ``prism_shuffle_cols``."""
+    X = _segment_aligned(X)
+    G, K = seg.shape[0], seg.shape[1] * 64
+    Y = torch.empty_like(X)
+    with torch.cuda.device(X.device):
+        _lib.check(_lib.lib().prism_shuffle_cols(_ptr(X), _ptr(Y), _ptr(seg), G, X.shape[0] // G, K, X.element_size(),
+                                                 _stream_ptr(X.device)))
+    return Y
+
+
+def shuffle_fold_r(R, inv_seg):
+    """R (G * 16, K) -> R64 (G * 64, K), 16-bit, through ``prism_shuffle_fold_r``."""
+    R = _segment_aligned(R)
+    G, K = inv_seg.shape[0], inv_seg.shape[1] * 64
+    R64 = torch.empty(G * 64, K, dtype=R.dtype, device=R.device)
+    with torch.cuda.device(R.device):
+        _lib.check(_lib.lib().prism_shuffle_fold_r(_ptr(R), _ptr(R64), _ptr(inv_seg), G, K, _stream_ptr(R.device)))
+    return R64
+
+
+def shuffle_unfold_r(dR64, perm_seg):
+    """Adjoint of ``shuffle_fold_r``, 16- or 32-bit, through ``prism_shuffle_unfold_r``."""
+    dR64 = _segment_aligned(dR64)
+    G, K = perm_seg.shape[0], perm_seg.shape[1] * 64
+    dR = torch.empty(G * 16, K, dtype=dR64.dtype, device=dR64.device)
+    with torch.cuda.device(dR.device):
+        _lib.check(_lib.lib().prism_shuffle_unfold_r(_ptr(dR64), _ptr(dR), _ptr(perm_seg), G, K, dR64.element_size(),
+                                                     _stream_ptr(dR.device)))
+    return dR
+
+
 def _out_buffer(out, shape, dtype, device, name):
     """``out`` if given (a contiguous tensor of that shape and dtype, e.g. a view of a gradient staging
     buffer that other GPUs read), else a new tensor."""

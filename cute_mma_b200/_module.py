@@ -130,6 +130,57 @@ def _cayley_backward(ctx, dR):
 _cayley_op.register_autograd(_cayley_backward, setup_context=_cayley_setup)
 
 
+# The copies of the input shuffle.  Each takes its own table and that of its adjoint, which its gradient uses.
+@torch.library.custom_op("prism_b200::shuffle_cols", mutates_args=())
+def _shuffle_cols_op(X: torch.Tensor, seg: torch.Tensor, adjoint_seg: torch.Tensor) -> torch.Tensor:
+    return F.shuffle_cols(X, seg)
+
+
+@_shuffle_cols_op.register_fake
+def _(X, seg, adjoint_seg):
+    return X.new_empty(X.shape)
+
+
+@torch.library.custom_op("prism_b200::shuffle_fold_r", mutates_args=())
+def _shuffle_fold_r_op(R: torch.Tensor, inv_seg: torch.Tensor, perm_seg: torch.Tensor) -> torch.Tensor:
+    return F.shuffle_fold_r(R, inv_seg)
+
+
+@_shuffle_fold_r_op.register_fake
+def _(R, inv_seg, perm_seg):
+    return R.new_empty(R.shape[0] * 4, R.shape[1])
+
+
+@torch.library.custom_op("prism_b200::shuffle_unfold_r", mutates_args=())
+def _shuffle_unfold_r_op(dR64: torch.Tensor, perm_seg: torch.Tensor, inv_seg: torch.Tensor) -> torch.Tensor:
+    return F.shuffle_unfold_r(dR64, perm_seg)
+
+
+@_shuffle_unfold_r_op.register_fake
+def _(dR64, perm_seg, inv_seg):
+    return dR64.new_empty(dR64.shape[0] // 4, dR64.shape[1])
+
+
+def _shuffle_setup(ctx, inputs, output):
+    ctx.save_for_backward(inputs[1], inputs[2])
+
+
+def _shuffle_grad(adjoint):
+    def backward(ctx, grad):
+        seg, adjoint_seg = ctx.saved_tensors
+        return adjoint(grad, adjoint_seg, seg), None, None
+    return backward
+
+
+_shuffle_cols_op.register_autograd(_shuffle_grad(_shuffle_cols_op), setup_context=_shuffle_setup)
+_shuffle_fold_r_op.register_autograd(_shuffle_grad(_shuffle_unfold_r_op), setup_context=_shuffle_setup)
+_shuffle_unfold_r_op.register_autograd(_shuffle_grad(_shuffle_fold_r_op), setup_context=_shuffle_setup)
+
+
+class shuffle_ops:
+    cols, fold_r, unfold_r = _shuffle_cols_op, _shuffle_fold_r_op, _shuffle_unfold_r_op
+
+
 def _setup_context(ctx, inputs, output):
     A, B, R, bias, group_size, reconn_sz, activation, bwd_scale, internal_bias, dropout_seeds, dropout_p = inputs
     ctx.save_for_backward(A, B, R, *(() if internal_bias is None else (internal_bias,)))

@@ -78,6 +78,15 @@ def shuffle_perm(shuffle_masks: torch.Tensor, K: int, reconn_sz: int) -> torch.T
     return perm.reshape(G, K)
 
 
+_NATIVE = (torch.float16, torch.bfloat16, torch.float32)
+
+
+def _ops():
+    """The copy kernels as differentiable custom ops (registered beside the layer's)."""
+    from . import _module
+    return _module.shuffle_ops
+
+
 class ShuffleFold:
     """Index maps of one set of masks (built once per module, or per functional call)."""
 
@@ -95,9 +104,20 @@ class ShuffleFold:
         self.inv = inv.to(device)
         self.inv_in_chunk = (inv.view(G, n_chunks, 64) % 64).to(device)       # the same, inside its chunk
         self.perm_in_chunk = (perm.view(G, n_chunks, 64) % 64).to(device)
+        # the same per segment of two features, as the copy kernels take it
+        self.inv_seg = (self.inv_in_chunk[:, :, ::2] // 2).to(torch.uint8).contiguous()
+        self.perm_seg = (self.perm_in_chunk[:, :, ::2] // 2).to(torch.uint8).contiguous()
+
+    def _native(self, X: torch.Tensor, rows: int, sizes=(2,)) -> bool:
+        """Whether the library's copy kernels take X: on this fold's GPU, elements of 2 (or 4) bytes, whole rows;
+        everything else goes through the index operations."""
+        return (X.is_cuda and X.device == self.inv_seg.device and X.dtype in _NATIVE and X.element_size() in sizes
+                and X.is_contiguous() and X.shape == (self.G * rows, self.K) and self.G <= 65535 and self.n_chunks <= 65535)
 
     def fold_R(self, R: torch.Tensor) -> torch.Tensor:
         """``R (G * 16, K)`` -> ``R64 (G * 64, K)``: per chunk ``P . blockdiag(R) . P^T`` (differentiable)."""
+        if self._native(R, 16):
+            return _ops().fold_r(R, self.inv_seg, self.perm_seg)
         G, nc = self.G, self.n_chunks
         Rb = R.view(G, 16, nc, 4, 16).permute(0, 2, 3, 1, 4)                  # g, chunk, block, i, j
         bd = R.new_zeros(G, nc, 4, 16, 4, 16)
@@ -110,6 +130,8 @@ class ShuffleFold:
 
     def unfold_dR(self, dR64: torch.Tensor) -> torch.Tensor:
         """Gradient of ``fold_R``: the diagonal 16 x 16 blocks of ``P^T . dR64 . P``."""
+        if self._native(dR64, 64, (2, 4)):
+            return _ops().unfold_r(dR64, self.perm_seg, self.inv_seg)
         G, nc = self.G, self.n_chunks
         d = dR64.view(G, 64, nc, 64).permute(0, 2, 1, 3)
         idx = self.perm_in_chunk
@@ -120,9 +142,13 @@ class ShuffleFold:
 
     def fold_cols(self, X: torch.Tensor, rows_per_group: int) -> torch.Tensor:
         """Columns of a per-group matrix (``B``: ``(G * gs, K)``; internal bias: ``(G, K)``) into physical order."""
+        if self._native(X, rows_per_group, (2, 4)):
+            return _ops().cols(X, self.inv_seg, self.perm_seg)
         Xg = X.view(self.G, rows_per_group, self.K)
         return Xg.gather(2, self.inv[:, None, :].expand(-1, rows_per_group, -1)).reshape(X.shape).contiguous()
 
     def unfold_cols(self, dX: torch.Tensor, rows_per_group: int) -> torch.Tensor:
+        if self._native(dX, rows_per_group, (2, 4)):
+            return _ops().cols(dX, self.perm_seg, self.inv_seg)
         dXg = dX.view(self.G, rows_per_group, self.K)
         return dXg.gather(2, self.perm[:, None, :].expand(-1, rows_per_group, -1)).reshape(dX.shape).contiguous()

@@ -165,6 +165,18 @@ int prism_cayley(const void* M, void* R, int n_groups, int K, int reconn_sz, int
 int prism_cayley_bwd(const void* M, const void* dR, void* dM, int n_groups, int K, int reconn_sz, int dtype,
                      long long ldm, long long lddr, long long lddm, void* stream);
 
+/* Copies of the input shuffle (PrismLinear(input_shuffle=True); the reference gathers a permuted copy of A per
+ * group instead, torch_ext/prism_fwd_torch.cu:122-139).  A permutation moves segments of two neighbouring features
+ * inside chunks of 64: seg [G, K/64, 32] (bytes, values below 32).
+ * prism_shuffle_cols: X, Y [G * rows_per_group, K], elements of esize 2 or 4 bytes: segment i of a row's chunk of Y is
+ * segment seg[g, chunk, i] of X's.
+ * prism_shuffle_fold_r: R [G*16, K] -> R64 [G*64, K] (16-bit): the chunk's four 16 x 16 blocks as one 64 x 64 block in
+ * physical feature order, inv_seg = physical -> logical.  prism_shuffle_unfold_r: its adjoint, seg = logical -> physical. */
+int prism_shuffle_cols(const void* X, void* Y, const unsigned char* seg, int G, int rows_per_group, int K, int esize,
+                       void* stream);
+int prism_shuffle_fold_r(const void* R, void* R64, const unsigned char* inv_seg, int G, int K, void* stream);
+int prism_shuffle_unfold_r(const void* dR64, void* dR, const unsigned char* seg, int G, int K, int esize, void* stream);
+
 /* Sum of gradient buffers over the GPUs of one box, over peer memory: the exchange step of token-sharded
  * training (the reference leaves it to DistributedDataParallel's all-reduce, integration/train.py:130-145,
  * 299-300).  in_ptrs / out_ptrs: HOST arrays of `world` device pointers -- every rank's fp32 buffer of n

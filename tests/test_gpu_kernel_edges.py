@@ -57,7 +57,7 @@ def test_widened_and_halved_rotation(K, rs):
 
 
 @pytest.mark.parametrize("M,K,N,gs", [(128, 256, 256, 256),       # one token block: never split
-                                      (129, 264, 512, 256),       # two blocks, features past the first pair
+                                      (129, 272, 512, 256),       # two blocks, features past the first pair
                                       (2200, 256, 256, 128),      # few tiles: split as often as it pays
                                       (4096, 1024, 4096, 256)])   # 64 tiles: one wave, not split
 @pytest.mark.parametrize("out", [None, torch.float32])
@@ -68,3 +68,27 @@ def test_split_plan_of_db(M, K, N, gs, out):
     cp.check_device_status()
     ref = O.prism_backward(dC.float(), A.float(), B.float(), R.float(), gs, rs, act)[2]
     assert dB.dtype == (out or dt) and O.rel_err(dB.float(), ref) < TOL
+
+
+@pytest.mark.parametrize("G,K,rows", [(1, 64, 1), (3, 192, 33), (5, 1088, 8)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_shuffle_copies_are_the_index_operations(G, K, rows, dt):
+    """The copy kernels against the index operations of the same fold on the CPU: bit for bit, adjoints included; a matrix
+    that starts in the middle of a segment is taken too."""
+    from cute_mma_b200 import _shuffle as S
+    masks, _ = S.build_shuffle_masks(K, G * 32, 32, 16)
+    masks = masks if G > 1 else masks + 0x5A3C   # a single group is the identity otherwise
+    cpu, gpu = S.ShuffleFold(masks, K, 32, 16, "cpu"), S.ShuffleFold(masks, K, 32, 16, torch.device(DEV, 0))
+    X, D64 = torch.randn(G * rows, K).to(dt), torch.randn(G * 64, K).to(dt)
+    off = torch.empty(G * rows * K + 1, dtype=dt, device=DEV)[1:].view(G * rows, K).copy_(X)
+    for Y in (X.to(DEV), off):
+        assert torch.equal(gpu.fold_cols(Y, rows).cpu(), cpu.fold_cols(X, rows))
+        assert torch.equal(gpu.unfold_cols(Y, rows).cpu(), cpu.unfold_cols(X, rows))
+    assert torch.equal(gpu.unfold_dR(D64.to(DEV)).cpu(), cpu.unfold_dR(D64))
+    R = torch.randn(G * 16, K).to(dt)
+    r_gpu, r_cpu = R.to(DEV).requires_grad_(), R.clone().requires_grad_()
+    out, ref = gpu.fold_R(r_gpu), cpu.fold_R(r_cpu)
+    assert torch.equal(out.detach().cpu(), ref.detach())
+    out.backward(D64.to(DEV))
+    ref.backward(D64)
+    assert torch.equal(r_gpu.grad.cpu(), r_cpu.grad)
