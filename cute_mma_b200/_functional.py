@@ -383,6 +383,17 @@ def shuffle_unfold_r(dR64, perm_seg):
     return dR
 
 
+_MASK_BYTES_MAX = 1 << 30   # beyond this the dB kernel hashes again instead
+
+
+def _dropout_mask(seeds, M, N, K, group_size):
+    """Scratch in which the dA+dR kernel leaves the dropout mask for the dB kernel of the same backward, or None."""
+    if seeds is None:
+        return None
+    nbytes = _lib.lib().prism_dropout_mask_bytes(M, N, K, group_size)
+    return torch.empty(nbytes // 4, dtype=torch.int32, device=seeds.device) if 0 < nbytes <= _MASK_BYTES_MAX else None
+
+
 def _out_buffer(out, shape, dtype, device, name):
     """``out`` if given (a contiguous tensor of that shape and dtype, e.g. a view of a gradient staging
     buffer that other GPUs read), else a new tensor."""
@@ -394,7 +405,7 @@ def _out_buffer(out, shape, dtype, device, name):
 
 
 def _backward_db(dC, A, R, group_size, reconn_sz, gate, dc_scale=1.0, tile_cfg=None, out_dtype=None,
-                 internal_bias=None, dropout_seeds=None, dropout_p=0.0, dB_out=None):
+                 internal_bias=None, dropout_seeds=None, dropout_p=0.0, dB_out=None, dropout_mask=None):
     """dB = dc_scale * dC^T . H  through ``prism_bwd_db`` (H recomputed on chip); with
     ``out_dtype=torch.float32`` the kernel's fp32 sums are returned unrounded.  ``dB_out``: write there."""
     M, K = A.shape
@@ -408,16 +419,16 @@ def _backward_db(dC, A, R, group_size, reconn_sz, gate, dc_scale=1.0, tile_cfg=N
     with torch.cuda.device(A.device):
         need = L.prism_workspace_bytes(KIND_BWD_DB, M, N, K, group_size, reconn_sz, dt, cfg_arr)
         ws = _workspace.get(A.device, need)
-        _lib.check(L.prism_bwd_db(
+        _lib.check(L.prism_bwd_db_mask(
             ctypes.c_void_p(dC.data_ptr()), ctypes.c_void_p(A.data_ptr()), ctypes.c_void_p(R.data_ptr()),
             _ptr(internal_bias), ctypes.c_void_p(dB.data_ptr()), M, N, K, group_size, reconn_sz, dt, gate, out_code,
             ctypes.c_float(dc_scale), dC.stride(0), A.stride(0), R.stride(0), dB.stride(0),
-            _ptr(dropout_seeds), ctypes.c_float(dropout_p if dropout_seeds is not None else 0.0), cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
+            _ptr(dropout_seeds), ctypes.c_float(dropout_p if dropout_seeds is not None else 0.0), _ptr(dropout_mask), cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
     return dB
 
 
 def _backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, dc_scale=1.0, tile_cfg=None, dR_dtype=None,
-                   internal_bias=None, dropout_seeds=None, dropout_p=0.0, dR_out=None):
+                   internal_bias=None, dropout_seeds=None, dropout_p=0.0, dR_out=None, dropout_mask=None):
     """(dA, dR), both scaled by ``dc_scale``, through ``prism_bwd_dadr``; with
     ``dR_dtype=torch.float32`` the fp32 sums of the dR reduction are returned unrounded.  With an
     ``internal_bias`` the result is ``(dA, dR, d_internal_bias)``."""
@@ -435,13 +446,13 @@ def _backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, dc_scale=1.0, tile_
         kind = KIND_BWD_DADR_IB if internal_bias is not None else KIND_BWD_DADR
         need = L.prism_workspace_bytes(kind, M, N, K, group_size, reconn_sz, dt, cfg_arr)
         ws = _workspace.get(A.device, need)
-        _lib.check(L.prism_bwd_dadr(
+        _lib.check(L.prism_bwd_dadr_mask(
             ctypes.c_void_p(dC.data_ptr()), ctypes.c_void_p(A.data_ptr()), ctypes.c_void_p(B.data_ptr()),
             ctypes.c_void_p(R.data_ptr()), _ptr(internal_bias), ctypes.c_void_p(dA.data_ptr()),
             ctypes.c_void_p(dR.data_ptr()), _ptr(d_ib),
             M, N, K, group_size, reconn_sz, dt, gate, dr_code, ctypes.c_float(dc_scale),
             dC.stride(0), A.stride(0), B.stride(0), R.stride(0), dA.stride(0), dR.stride(0),
-            _ptr(dropout_seeds), ctypes.c_float(dropout_p if dropout_seeds is not None else 0.0), cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
+            _ptr(dropout_seeds), ctypes.c_float(dropout_p if dropout_seeds is not None else 0.0), _ptr(dropout_mask), cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
     if internal_bias is not None:
         return dA, dR, d_ib
     return dA, dR
@@ -486,10 +497,11 @@ def backward(dC, A, B, R, group_size: int = 256, reconn_sz: int = 8, backend=Non
     if gate and dropout_seeds is not None and dropout_p > 0.0:
         _check_dropout(dropout_p, reconn_sz)
         seeds = _check_seeds(dropout_seeds, A, N // group_size)
+    mask = _dropout_mask(seeds, M, N, K, group_size)
     out = _backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_dadr, dR_dtype, internal_bias,
-                         seeds, dropout_p)
+                         seeds, dropout_p, dropout_mask=mask)
     dB = (_backward_db(dC, A, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_db, dB_dtype, internal_bias,
-                       seeds, dropout_p) if gate else None)
+                       seeds, dropout_p, dropout_mask=mask) if gate else None)
     return out[0], out[1], dB, (out[2] if internal_bias is not None else None)
 
 

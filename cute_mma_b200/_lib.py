@@ -28,7 +28,7 @@ NVCC_FLAGS = [
 # every symbol include/prism_b200.h declares
 EXPORTS = [
     "prism_fwd", "prism_fwd_dropout", "prism_fwd_noalloc", "prism_bwd_dadr", "prism_bwd_db", "prism_dbias", "prism_fold_weight", "prism_cayley", "prism_cayley_bwd", "prism_peer_reduce",
-    "prism_shuffle_cols", "prism_shuffle_fold_r", "prism_shuffle_unfold_r", "prism_workspace_bytes",
+    "prism_bwd_dadr_mask", "prism_bwd_db_mask", "prism_dropout_mask_bytes", "prism_shuffle_cols", "prism_shuffle_fold_r", "prism_shuffle_unfold_r", "prism_workspace_bytes",
     "prism_status",
     "prism_last_error_string", "prism_abi_version", "prism_launch_count",
 ]
@@ -124,6 +124,14 @@ def lib() -> ctypes.CDLL:
                 L.prism_bwd_db.restype = i
                 L.prism_bwd_db.argtypes = [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, ctypes.c_float,
                                            ll, ll, ll, ll, vp, ctypes.c_float, ip, vp, sz, vp]
+            L.prism_bwd_dadr_mask.restype = i
+            L.prism_bwd_dadr_mask.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, ctypes.c_float,
+                                              ll, ll, ll, ll, ll, ll, vp, ctypes.c_float, vp, ip, vp, sz, vp]
+            L.prism_bwd_db_mask.restype = i
+            L.prism_bwd_db_mask.argtypes = [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, ctypes.c_float,
+                                            ll, ll, ll, ll, vp, ctypes.c_float, vp, ip, vp, sz, vp]
+            L.prism_dropout_mask_bytes.restype = sz
+            L.prism_dropout_mask_bytes.argtypes = [i, i, i, i]
             L.prism_dbias.restype = i
             L.prism_dbias.argtypes = [vp, vp, i, i, i, i, ll, vp, sz, vp]
             L.prism_fold_weight.restype = i

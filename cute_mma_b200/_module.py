@@ -73,15 +73,16 @@ def _prism_backward_op(dC: torch.Tensor, A: torch.Tensor, B: torch.Tensor, R: to
     A, B, R = A.contiguous(), B.contiguous(), R.contiguous()
     gate = F._gate_code(activation or None)
     ib = internal_bias.contiguous() if internal_bias is not None else None
+    mask = F._dropout_mask(dropout_seeds if need_dB and gate else None, A.shape[0], B.shape[0], A.shape[1], group_size)
     out = F._backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
-                           dropout_seeds=dropout_seeds, dropout_p=dropout_p)
+                           dropout_seeds=dropout_seeds, dropout_p=dropout_p, dropout_mask=mask)
     dA, dR = out[0], out[1]
     d_ib = out[2] if ib is not None else dC.new_empty(0)
     if not need_dB:
         dB = B.new_empty(0)
     elif gate:
         dB = F._backward_db(dC, A, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
-                            dropout_seeds=dropout_seeds, dropout_p=dropout_p)
+                            dropout_seeds=dropout_seeds, dropout_p=dropout_p, dropout_mask=mask)
     else:
         dB = torch.zeros_like(B)  # frozen-B contract of the reference's plain mode
     # the bias is added after the rescale point: its gradient is the plain column sum of dC

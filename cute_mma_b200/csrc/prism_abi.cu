@@ -218,6 +218,11 @@ static int check_dropout(const char* fn, const void* seeds, float p, int gate) {
   return PRISM_OK;
 }
 
+static int check_mask(const char* fn, const void* mask) {
+  if (reinterpret_cast<uintptr_t>(mask) % 4 != 0) return fail(PRISM_ERR_BAD_ARG, "%s: dropout_mask must be 4-byte aligned", fn);
+  return PRISM_OK;
+}
+
 static int check_ptr(const char* fn, const char* name, const void* p, long long ld, int min_ld) {
   if (p == nullptr) return fail(PRISM_ERR_BAD_ARG, "%s: %s is null", fn, name);
   if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return fail(PRISM_ERR_BAD_ARG, "%s: %s must be 16-byte aligned", fn, name);
@@ -280,6 +285,12 @@ extern "C" size_t prism_workspace_bytes(int kind, int M, int N, int K, int gs, i
     return bytes;
   }
   return bytes;
+}
+
+// words of 32 mask bits: one per thread of a gate task (16 tokens x 64 features), tasks ordered [group][token rows][features]
+extern "C" size_t prism_dropout_mask_bytes(int M, int N, int K, int gs) {
+  if (M <= 0 || N <= 0 || K <= 0 || gs <= 0) return 0;
+  return (size_t)(N / gs) * ((M + 127) / 128) * 8 * ((K + 63) / 64) * 32 * 4;
 }
 
 extern "C" int prism_status(void* workspace, void* stream) {
@@ -364,10 +375,10 @@ extern "C" int prism_fwd_dropout(const void* A, const void* B, const void* R, co
   return launch_fwd(a);
 }
 
-extern "C" int prism_bwd_db(const void* dC, const void* A, const void* R, const void* internal_bias, void* dB,
+extern "C" int prism_bwd_db_mask(const void* dC, const void* A, const void* R, const void* internal_bias, void* dB,
                             int M, int N, int K, int gs, int rs, int dtype, int gate, int db_dtype, float dc_scale,
                             long long lddc, long long lda, long long ldr, long long lddb,
-                            const long long* dropout_seeds, float dropout_p,
+                            const long long* dropout_seeds, float dropout_p, const void* dropout_mask,
                             const int* cfg, void* workspace, size_t workspace_bytes, void* stream) {
   const char* fn = "prism_bwd_db";
   int rc;
@@ -378,6 +389,7 @@ extern "C" int prism_bwd_db(const void* dC, const void* A, const void* R, const 
   if ((rc = check_ptr(fn, "dB", dB, lddb, K))) return rc;
   if ((rc = check_ib(fn, internal_bias, gate))) return rc;
   if ((rc = check_dropout(fn, dropout_seeds, dropout_p, gate))) return rc;
+  if ((rc = check_mask(fn, dropout_mask))) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (M == 0) {  // no tokens: the gradient is zero
     const size_t es = db_f32 ? 4 : 2;
@@ -393,6 +405,7 @@ extern "C" int prism_bwd_db(const void* dC, const void* A, const void* R, const 
 
   DbArgs a;
   a.dC = dC; a.A = A; a.dB = dB; a.ib = internal_bias; a.drop_seeds = dropout_seeds; a.drop_p = dropout_p;
+  a.drop_mask = reinterpret_cast<const uint32_t*>(dropout_mask);
   a.M = M; a.N = N; a.K = K; a.gs = gs; a.E = effective_block(rs);
   a.dtype = dtype; a.gate = gate; a.scale = dc_scale; a.out_f32 = db_f32;
   a.lddc = lddc; a.lda = lda; a.lddb = lddb;
@@ -414,11 +427,20 @@ extern "C" int prism_bwd_db(const void* dC, const void* A, const void* R, const 
   return launch_bwd_db(a);
 }
 
-extern "C" int prism_bwd_dadr(const void* dC, const void* A, const void* B, const void* R, const void* internal_bias,
+extern "C" int prism_bwd_db(const void* dC, const void* A, const void* R, const void* internal_bias, void* dB,
+                            int M, int N, int K, int gs, int rs, int dtype, int gate, int db_dtype, float dc_scale,
+                            long long lddc, long long lda, long long ldr, long long lddb,
+                            const long long* dropout_seeds, float dropout_p,
+                            const int* cfg, void* workspace, size_t workspace_bytes, void* stream) {
+  return prism_bwd_db_mask(dC, A, R, internal_bias, dB, M, N, K, gs, rs, dtype, gate, db_dtype, dc_scale, lddc, lda,
+                           ldr, lddb, dropout_seeds, dropout_p, nullptr, cfg, workspace, workspace_bytes, stream);
+}
+
+extern "C" int prism_bwd_dadr_mask(const void* dC, const void* A, const void* B, const void* R, const void* internal_bias,
                               void* dA, void* dR, void* d_internal_bias, int M, int N, int K, int gs, int rs, int dtype, int gate,
                               int dr_dtype, float dc_scale, long long lddc, long long lda, long long ldb,
                               long long ldr, long long ldda, long long lddr,
-                              const long long* dropout_seeds, float dropout_p, const int* cfg,
+                              const long long* dropout_seeds, float dropout_p, void* dropout_mask, const int* cfg,
                               void* workspace, size_t workspace_bytes, void* stream) {
   const char* fn = "prism_bwd_dadr";
   int rc;
@@ -429,6 +451,7 @@ extern "C" int prism_bwd_dadr(const void* dC, const void* A, const void* B, cons
   if ((rc = check_ptr(fn, "dR", dR, lddr, K))) return rc;
   if ((rc = check_ib(fn, internal_bias, gate))) return rc;
   if ((rc = check_dropout(fn, dropout_seeds, dropout_p, gate))) return rc;
+  if ((rc = check_mask(fn, dropout_mask))) return rc;
   const bool with_ib = internal_bias != nullptr;
   if (with_ib && d_internal_bias == nullptr) return fail(PRISM_ERR_BAD_ARG, "%s: d_internal_bias is null", fn);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
@@ -449,7 +472,7 @@ extern "C" int prism_bwd_dadr(const void* dC, const void* A, const void* B, cons
 
   DadrArgs a;
   a.dC = dC; a.A = A; a.B = B; a.dA = dA; a.dR = dR; a.ib = internal_bias; a.d_ib = d_internal_bias;
-  a.drop_seeds = dropout_seeds; a.drop_p = dropout_p;
+  a.drop_seeds = dropout_seeds; a.drop_p = dropout_p; a.drop_mask = reinterpret_cast<uint32_t*>(dropout_mask);
   a.M = M; a.N = N; a.K = K; a.gs = gs; a.rs = rs; a.E = effective_block(rs);
   a.dtype = dtype; a.gate = gate; a.scale = dc_scale; a.dr_f32 = dr_f32;
   a.lddc = lddc; a.lda = lda; a.ldb = ldb; a.ldda = ldda; a.lddr = lddr;
@@ -474,6 +497,17 @@ extern "C" int prism_bwd_dadr(const void* dC, const void* A, const void* B, cons
   a.err = reinterpret_cast<int*>(workspace);
   a.stream = s;
   return launch_bwd_dadr(a);
+}
+
+extern "C" int prism_bwd_dadr(const void* dC, const void* A, const void* B, const void* R, const void* internal_bias,
+                              void* dA, void* dR, void* d_internal_bias, int M, int N, int K, int gs, int rs, int dtype, int gate,
+                              int dr_dtype, float dc_scale, long long lddc, long long lda, long long ldb,
+                              long long ldr, long long ldda, long long lddr,
+                              const long long* dropout_seeds, float dropout_p, const int* cfg,
+                              void* workspace, size_t workspace_bytes, void* stream) {
+  return prism_bwd_dadr_mask(dC, A, B, R, internal_bias, dA, dR, d_internal_bias, M, N, K, gs, rs, dtype, gate,
+                             dr_dtype, dc_scale, lddc, lda, ldb, ldr, ldda, lddr, dropout_seeds, dropout_p, nullptr,
+                             cfg, workspace, workspace_bytes, stream);
 }
 
 extern "C" int prism_dbias(const void* dC, void* dbias, int M, int N, int dtype, int dbias_dtype, long long lddc,

@@ -167,7 +167,7 @@ int launch_bwd_dadr(const DadrArgs& a) {
 
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "bwd_dadr: dropout needs reconn_sz 8 or 16");
-  x.drop_seeds = a.drop_seeds; x.drop_p = a.drop_p; x.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
+  x.drop_seeds = a.drop_seeds; x.drop_thr = drop_threshold(a.drop_p); x.drop_mask = a.drop_mask; x.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   DadrKernel kern = (a.dtype == DT_BF16) ? dadr_kernel_bf16(a.gate, a.E, ib, drop) : dadr_kernel_f16(a.gate, a.E, ib, drop);
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_dadr"))) return rc;
   dim3 grid(2 * (p.n_main + p.n_extra), 1, 1);   // the two CTAs of a pair are neighbours

@@ -83,7 +83,9 @@ struct DadrParams {
 // fields inside DadrParams the instance without either (the benchmarked one) compiled to more spills.
 struct DadrExtra {
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
-  float drop_p, drop_inv_keep;
+  uint32_t drop_thr;   // see drop_threshold
+  float drop_inv_keep;
+  uint32_t* drop_mask;   // the mask words are also left here for the dB kernel (prism_dropout_mask_bytes), or null
   const void* ib;      // internal bias [G, K] (gated modes, IB kernels) or null
   float* partial_ib;   // [2*runs][G][K] fp32: column sums of dS of the main CTAs
   float* partial_ib_x; // [2*n_extra][slots][G][128] fp32: ... of the extra pairs' CTAs
@@ -235,7 +237,7 @@ __device__ __forceinline__ float* dadr_unit_ib(const DadrParams& p, const DadrEx
 // the tokens (the bias gradient) leave through a second set of per-CTA fp32 buffers: every gate warp
 // sums its 16 token rows with shuffles, the 8 warps of a 64-feature chunk meet in shared memory, are
 // added in a fixed order, and one thread per column stores (first tile) or adds (later tiles).
-// DROP: hash dropout (see DropCtx): dH is multiplied by the forward's mask before it is used.
+// DROP: hash dropout (see drop_mask32): dH is multiplied by the forward's mask before it is used.
 template <int DT, int GATE, int E, bool IB, bool DROP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(dadr::kThreads, 1)
 prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmRr,
@@ -530,20 +532,19 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!mbar_wait(&bars->a_full, tile_iter & 1)) { ok = false; break; }
       for (int g = 0; g < G && ok; ++g, ++gg) {
         const uint32_t hb = gg & 1, ph = (gg >> 1) & 1;
+        uint32_t mask = 0;
+        if (DROP && kGated) {   // before the waits: the hash needs indices only
+          mask = drop_mask32(drop_group_hash(ex.drop_seeds, g),
+                             (uint64_t)(mt * 128 + (int)r0 + (lane >> 2)) * p.K + f0 + ch * 64 + 2 * (lane & 3), 8ull * p.K, ex.drop_thr);
+          if (ex.drop_mask != nullptr && mt < p.n_mtiles && f0 + ch * 64 < p.K)
+            ex.drop_mask[(((long long)g * p.n_mtiles * 8 + mt * 8 + (int)(r0 >> 4)) * ((p.K + 63) >> 6) + (f0 >> 6) + ch) * 32 + lane] = mask;
+        }
         if (kGated) {
           if (!mbar_wait(&bars->s_full, gg & 1)) { ok = false; break; }
         }
         if (!mbar_wait(&bars->dh_full[hb], ph)) { ok = false; break; }
         if (!mbar_wait(&bars->ds_empty[hb], ph ^ 1)) { ok = false; break; }
         tc_fence_after_sync();
-        DropCtx dctx;
-        if (DROP && kGated) {
-          dctx.h1 = drop_group_hash(ex.drop_seeds, g);
-          dctx.base = (long long)(mt * 128 + (int)r0 + (lane >> 2)) * p.K + f0 + ch * 64 + 2 * (lane & 3);
-          dctx.row8 = 8ll * p.K;
-          dctx.p = ex.drop_p;
-          dctx.inv_keep = ex.drop_inv_keep;
-        }
         const uint32_t tileDS = smem_u32(smemDS + hb * 2 * kTile + ch * kTile);
         const uint32_t tdh = tmem_base + lane_base + kDhCol0 + hb * 128 + ch * 64;
         const uint32_t ts = tmem_base + lane_base + kSCol0 + ch * 64;
@@ -596,8 +597,8 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               // pair e of the fragment: (row, cols) as in the accumulator layout; e >> 1 selects columns + 8
               float x0 = __uint_as_float(dh[i][2 * e]), x1 = __uint_as_float(dh[i][2 * e + 1]);
               if (DROP && kGated) {
-                x0 *= dctx.mul(e & 1, pc * 16 + (e >> 1) * 8);
-                x1 *= dctx.mul(e & 1, pc * 16 + (e >> 1) * 8 + 1);
+                x0 *= drop_mul(mask, pc * 8 + 2 * e, ex.drop_inv_keep);
+                x1 *= drop_mul(mask, pc * 8 + 2 * e + 1, ex.drop_inv_keep);
               }
               if (kGated) {
                 float* d = (e >> 1) ? d1 : d0;

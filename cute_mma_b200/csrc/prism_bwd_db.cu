@@ -52,7 +52,10 @@ struct DbParams {
   float scale;
   const void* ib;     // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
-  float drop_p, drop_inv_keep;
+  uint32_t drop_thr;   // see drop_threshold
+  float drop_inv_keep;
+  const uint32_t* drop_mask;   // the masks as the dA+dR kernel left them (prism_dropout_mask_bytes), or null: hash again
+  int n_k64;
   void* dB;
   long long lddb;
   float* partial;     // [splits][part_rows][K] when splits > 1
@@ -233,18 +236,20 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     bool ok = true;
     Ring rs(p.ns);
     for (int j = 0; j < nb && ok; ++j, rs.next()) {
+      uint32_t mask = 0;
+      if (DROP) {   // before the wait: neither needs anything that is being loaded
+        if (p.drop_mask != nullptr) {
+          const long long m16 = (long long)(tb0 + j) * 8 + (int)(r0 >> 4);
+          mask = kvalid > 0 ? __ldg(p.drop_mask + (((long long)g * p.n_tokblocks * 8 + m16) * p.n_k64 + (kcol >> 6)) * 32 + lane) : 0u;
+        } else {
+          mask = drop_mask32(drop_h1, (uint64_t)((tb0 + j) * 128 + (int)r0 + (lane >> 2)) * p.K + kcol + 2 * (lane & 3),
+                             8ull * p.K, p.drop_thr);
+        }
+      }
       if (!mbar_wait(&bars->s_full, j & 1)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t tile = smem_u32(smemSt + rs.idx * p.stage_bytes + ft * kTile);
-      DropCtx dc;
-      if (DROP) {
-        dc.h1 = drop_h1;
-        dc.base = (long long)((tb0 + j) * 128 + (int)r0 + (lane >> 2)) * p.K + kcol + 2 * (lane & 3);
-        dc.row8 = 8ll * p.K;
-        dc.p = p.drop_p;
-        dc.inv_keep = p.drop_inv_keep;
-      }
-      gate_rows16_tmem_smem<DT, GATE, E, DROP>(s_tmem, 2 * E, tile, r0, lane, s_free_addr, ib, kvalid, &dc);
+      gate_rows16_tmem_smem<DT, GATE, E, DROP>(s_tmem, 2 * E, tile, r0, lane, s_free_addr, ib, kvalid, mask, p.drop_inv_keep);
       fence_proxy_async_smem();   // H was written by the generic proxy, the MMA reads it through the async proxy
       tc_fence_before_sync();
       __syncwarp();
@@ -369,7 +374,7 @@ int launch_bwd_db(const DbArgs& a) {
   p.r_tile_bytes = ((a.E * 128) + 1023) / 1024 * 1024;
   p.scale = a.scale; p.out_f32 = a.out_f32; p.ib = a.ib;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
-  p.drop_seeds = a.drop_seeds; p.drop_p = a.drop_p; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
+  p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_mask = a.drop_mask; p.n_k64 = (a.K + 63) / 64; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "bwd_db: dropout needs reconn_sz 8 or 16");
   p.dB = a.dB; p.lddb = a.lddb; p.partial = a.partial; p.err = a.err;
   if ((a.plan.splits > 1 || a.plan.tail_rows > 0) && a.partial == nullptr)

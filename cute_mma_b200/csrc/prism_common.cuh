@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "../../include/prism_b200.h"
@@ -661,18 +662,38 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
   return x ^ (x >> 31);
 }
-struct DropCtx {
-  uint64_t h1;       // splitmix64(seed_g + 0xdeadbeef)
-  long long base;    // m*K + k of this thread's first element: row r0 + lane/4 of the warp, column 2 (lane%4) of the chunk
-  long long row8;    // 8 * K: the thread's second row
-  float p, inv_keep;
-  // multiplier of the element `rsel` rows of 8 down and `col` columns to the right
-  __device__ __forceinline__ float mul(int rsel, int col) const {
-    const uint64_t h = splitmix64(h1 ^ splitmix64((uint64_t)(base + rsel * row8 + col)));
-    const float u = (float)((h >> 40) & 0xFFFFFFull) * (1.0f / 16777216.0f);
-    return u >= p ? inv_keep : 0.f;
+// The mask of one gate task, 16 rows x 64 columns of a warp, as one word per thread: bit pc * 8 + 2 e + i is element i of
+// pair e of piece pc of the fragment layout (row lane/4, + 8 for odd e; column 16 pc + 2 (lane%4) + i, + 8 for e >= 2).
+//   h1    splitmix64(seed_g + 0xdeadbeef)
+//   base  m*K + k of the thread's first element: row r0 + lane/4, column 2 (lane%4) of the chunk
+//   row8  8 * K: the thread's second row;  thr: see drop_threshold
+// The hash needs nothing but indices, so the gate warps form the word before they wait for their operands, while it
+// costs no registers beside them (hashing element by element inside the gate arithmetic spilled).  The comparison is on
+// whole numbers: u = n / 2^24 with n < 2^24, and u >= p exactly when n >= ceil(p 2^24), i.e. when the hash's upper word is
+// at least thr; the int -> float conversion this replaces runs on the special-function pipe, which the gate's tanh needs.
+// splitmix64's last shift (x ^ x >> 31) does not reach the upper 24 bits: the outer hash ends at its product.
+__device__ __forceinline__ uint32_t drop_mask32(uint64_t h1, uint64_t base, uint64_t row8, uint32_t thr) {
+  uint32_t mask = 0;
+#pragma unroll 1
+  for (int pc = 0; pc < 4; ++pc, base += 16) {
+    uint32_t b = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {   // j = 2 e + i
+      uint64_t x = (h1 ^ splitmix64(base + ((j & 2) ? row8 : 0) + (j & 1) + ((j & 4) ? 8 : 0))) + 0x9e3779b97f4a7c15ull;
+      x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+      x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+      if ((uint32_t)(x >> 32) >= thr) b |= 1u << j;
+    }
+    mask |= b << (8 * pc);
   }
-};
+  return mask;
+}
+// multiplier of the element with mask bit `bit`
+__device__ __forceinline__ float drop_mul(uint32_t mask, int bit, float inv_keep) {
+  return (mask & (1u << bit)) ? inv_keep : 0.f;
+}
+// p in [0, 1) as the kernels compare it; p 2^24 and its ceiling are exact in fp32.
+inline uint32_t drop_threshold(float p) { return (uint32_t)ceilf(p * 16777216.f) << 8; }
 __device__ __forceinline__ uint64_t drop_group_hash(const long long* seeds, int g) {
   return splitmix64((uint64_t)__ldg(seeds + g) + 0xdeadbeefull);
 }
@@ -746,11 +767,11 @@ __device__ __forceinline__ void add_internal_bias(uint32_t (&s)[4][8], const uin
 // and is starved while a burst of tcgen05.mma runs (measured: 13x slower), which would serialise
 // the gate warps with the dense product.
 // ib / kvalid: internal bias of the chunk (see add_internal_bias), or null.
-// DROP / drop: hash dropout of H (see DropCtx).
+// DROP / mask / inv_keep: hash dropout of H (see drop_mask32).
 template <int DT, int GATE, bool DROP = false>
 __device__ __forceinline__ void gate_rows16_tmem(uint32_t s_tmem, uint32_t tile, uint32_t r0, int lane,
                                                  uint32_t h_tmem, const uint16_t* ib = nullptr, int kvalid = 64,
-                                                 const DropCtx* drop = nullptr) {
+                                                 uint32_t mask = 0u, float inv_keep = 1.f) {
   const uint32_t mat = lane >> 3, l8 = lane & 7;
   const uint32_t a_row = r0 + l8 + (mat & 1) * 8;
   uint32_t s[4][8], af[4][4], h[4][4];
@@ -772,8 +793,8 @@ __device__ __forceinline__ void gate_rows16_tmem(uint32_t s_tmem, uint32_t tile,
       // pair e: row r (e even) or r + 8 (e odd), columns pc*16 + 2(lane%4) + {0,1}, eight further on for e >= 2
       float m0 = 1.f, m1 = 1.f;
       if (DROP && GATE != GATE_NONE) {
-        m0 = drop->mul(e & 1, pc * 16 + (e >> 1) * 8);
-        m1 = drop->mul(e & 1, pc * 16 + (e >> 1) * 8 + 1);
+        m0 = drop_mul(mask, pc * 8 + 2 * e, inv_keep);
+        m1 = drop_mul(mask, pc * 8 + 2 * e + 1, inv_keep);
       }
       h[pc][e] = gate_pair<DT, GATE, (PRISM_FWD_CVT_HW != 0) && GATE != GATE_NONE, DROP>(
           af[pc][e], __uint_as_float(s[pc][2 * e]), __uint_as_float(s[pc][2 * e + 1]), m0, m1);
@@ -793,7 +814,7 @@ __device__ __forceinline__ void gate_rows16_tmem(uint32_t s_tmem, uint32_t tile,
 template <int DT, int GATE, int E, bool DROP = false>
 __device__ __forceinline__ void gate_rows16_tmem_smem(uint32_t s_tmem, uint32_t blk_stride, uint32_t tile, uint32_t r0,
                                                       int lane, uint32_t s_free, const uint16_t* ib = nullptr,
-                                                      int kvalid = 64, const DropCtx* drop = nullptr,
+                                                      int kvalid = 64, uint32_t mask = 0u, float inv_keep = 1.f,
                                                       uint32_t h_tile = 0, uint32_t h_r0 = 0) {
   constexpr int KS = E / 16;
   const uint32_t mat = lane >> 3, l8 = lane & 7;
@@ -824,8 +845,8 @@ __device__ __forceinline__ void gate_rows16_tmem_smem(uint32_t s_tmem, uint32_t 
     for (int e = 0; e < 4; ++e) {
       float m0 = 1.f, m1 = 1.f;
       if (DROP && GATE != GATE_NONE) {
-        m0 = drop->mul(e & 1, pc * 16 + (e >> 1) * 8);
-        m1 = drop->mul(e & 1, pc * 16 + (e >> 1) * 8 + 1);
+        m0 = drop_mul(mask, pc * 8 + 2 * e, inv_keep);
+        m1 = drop_mul(mask, pc * 8 + 2 * e + 1, inv_keep);
       }
       h[pc][e] = gate_pair<DT, GATE, (PRISM_DB_CVT_HW != 0) && GATE != GATE_NONE, DROP>(
           af[pc][e], __uint_as_float(s[pc][2 * e]), __uint_as_float(s[pc][2 * e + 1]), m0, m1);

@@ -63,7 +63,8 @@ struct FwdParams {
   const void* bias;     // [N] or null
   const void* ib;       // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
-  float drop_p, drop_inv_keep;
+  uint32_t drop_thr;   // see drop_threshold
+  float drop_inv_keep;
   void* C;
   long long ldc;
   int* err;
@@ -322,21 +323,18 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (uint32_t j = group; j < total; j += kGateGroups, rs.next(), rs.next()) {
       const uint32_t slot = j & (kSlots - 1);
+      uint32_t mask = 0;
+      if (DROP)   // before the wait: the hash needs indices only
+        mask = drop_mask32(drop_group_hash(p.drop_seeds, gcur),
+                           (uint64_t)((mtcur * 2 + (int)rank) * 128 + (int)r0 + (lane >> 2)) * p.K + kc * 64 + 2 * (lane & 3),
+                           8ull * p.K, p.drop_thr);
       if (!mbar_wait(&bars->s_full[slot], (j / kSlots) & 1)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t s_tmem = tmem_base + (r0 << 16) + kSlotCol0 + slot * 64;
       if (track) {
         const uint16_t* ib = ibase != nullptr ? ibase + (long long)gcur * p.K + kc * 64 : nullptr;
-        DropCtx dc;
-        if (DROP) {
-          dc.h1 = drop_group_hash(p.drop_seeds, gcur);
-          dc.base = (long long)((mtcur * 2 + (int)rank) * 128 + (int)r0 + (lane >> 2)) * p.K + kc * 64 + 2 * (lane & 3);
-          dc.row8 = 8ll * p.K;
-          dc.p = p.drop_p;
-          dc.inv_keep = p.drop_inv_keep;
-        }
         gate_rows16_tmem<DT, GATE, DROP>(s_tmem, smem_u32(smemSt + rs.idx * p.stage_bytes), r0, lane, s_tmem, ib,
-                                         p.K - kc * 64, &dc);
+                                         p.K - kc * 64, mask, p.drop_inv_keep);
         kc += kGateGroups;
         if (kc >= nk) {
           while (kc >= nk) { kc -= nk; tg += n_clusters; }
@@ -461,7 +459,7 @@ int launch_fwd(const FwdArgs& a) {
   p.tma_store = (a.BN % 64 == 0) ? 1 : 0;
   p.bias = a.bias; p.ib = a.ib; p.C = a.C; p.ldc = a.ldc; p.err = a.err;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
-  p.drop_seeds = a.drop_seeds; p.drop_p = a.drop_p; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
+  p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "forward: dropout needs reconn_sz 8 or 16");
 
   const int budget = 227 * 1024 - 1024 - (int)sizeof(FwdBarriers) - 256 - fwd::kNumEpiWarps * (fwd::kEpiStageBytes + fwd::kEpiBiasBytes);

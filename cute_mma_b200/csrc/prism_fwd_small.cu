@@ -51,7 +51,8 @@ struct FwdSmallParams {
   const void* bias;
   const void* ib;      // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
-  float drop_p, drop_inv_keep;
+  uint32_t drop_thr;   // see drop_threshold
+  float drop_inv_keep;
   void* C;
   long long ldc;
   float* partial;      // [G][pmax][Mp][gs] fp32
@@ -247,20 +248,16 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       int g = u0 / p.nk, kc = u0 - g * p.nk;
       for (int i = 0; i < n; ++i, rs.next()) {
         const uint32_t slot = (uint32_t)i & 1u;
+        uint32_t mask = 0;
+        if (DROP)   // before the wait: the hash needs indices only
+          mask = drop_mask32(drop_group_hash(p.drop_seeds, g), (uint64_t)((int)r0 + (lane >> 2)) * p.K + kc * 64 + 2 * (lane & 3),
+                             8ull * p.K, p.drop_thr);
         if (!mbar_wait(&bars->s_full[slot], ((uint32_t)i >> 1) & 1)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t tile = smem_u32(smemSt + rs.idx * p.stage_bytes + p.a_off);
         const uint16_t* ib = ibase != nullptr ? ibase + (long long)g * p.K + kc * 64 : nullptr;
-        DropCtx dc;
-        if (DROP) {
-          dc.h1 = drop_group_hash(p.drop_seeds, g);
-          dc.base = (long long)((int)r0 + (lane >> 2)) * p.K + kc * 64 + 2 * (lane & 3);
-          dc.row8 = 8ll * p.K;
-          dc.p = p.drop_p;
-          dc.inv_keep = p.drop_inv_keep;
-        }
         gate_rows16_tmem_smem<DT, GATE, E, DROP>(tmem_base + (r0 << 16) + kSCol0 + slot * 64, E, tile, r0, lane,
-                                                 smem_u32(&bars->s_free[slot]), ib, p.K - kc * 64, &dc);
+                                                 smem_u32(&bars->s_free[slot]), ib, p.K - kc * 64, mask, p.drop_inv_keep);
         if (++kc == p.nk) { kc = 0; ++g; }
         fence_proxy_async_smem();   // H was written by the generic proxy, the MMA reads it through the async proxy
         tc_fence_before_sync();
@@ -384,7 +381,7 @@ int launch_fwd_small(const FwdArgs& a, void* scratch) {
   fwd_small_partition(p.G, p.nk, a.num_sms, &p.units, &p.ncta, &p.pmax);
   p.bias = a.bias; p.ib = a.ib; p.C = a.C; p.ldc = a.ldc; p.err = a.err;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
-  p.drop_seeds = a.drop_seeds; p.drop_p = a.drop_p; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
+  p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "forward: dropout needs reconn_sz 8 or 16");
   p.partial = reinterpret_cast<float*>(scratch);
   // stage: A tile (Mp rows), R tile, B tiles, each on a 1024-byte boundary (128-byte swizzle atoms)

@@ -55,6 +55,7 @@ struct DbArgs {
   const void* ib;     // internal bias [N/gs, K] (gated modes) or null
   const long long* drop_seeds;  // [N/gs] per-group dropout seeds, or null
   float drop_p;
+  const uint32_t* drop_mask;  // mask words of prism_bwd_dadr_mask for the same dropout, or null
   void* dB;           // [N, K], 16-bit like the inputs or fp32 (out_f32)
   int M, N, K, gs, E;
   int dtype, gate;
@@ -90,6 +91,7 @@ struct DadrArgs {
   const void* ib;     // internal bias [N/gs, K] (gated modes) or null
   const long long* drop_seeds;  // [N/gs] per-group dropout seeds, or null
   float drop_p;
+  uint32_t* drop_mask;  // receives the mask words (prism_dropout_mask_bytes), or null
   void* d_ib;         // its gradient [N/gs, K] (same dtype as the inputs), when ib is given
   float* partial_ib;  // fp32 column sums of dS per main CTA: [2*runs][N/gs][K]
   float* partial_ib_x;  // ... and per slab of the extra pairs' CTAs: [2*n_extra][slots][N/gs][128]

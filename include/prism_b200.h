@@ -139,6 +139,22 @@ int prism_bwd_db(const void* dC, const void* A, const void* R, const void* inter
                  const long long* dropout_seeds, float dropout_p,
                  const int* cfg, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The two backward calls of one training step with dropout form the same mask.  prism_bwd_dadr_mask also leaves it in
+ * dropout_mask (prism_dropout_mask_bytes bytes, one bit per element of H, or NULL) and prism_bwd_db_mask, called after it
+ * on the same stream with the same sizes, seeds and probability, reads it there instead of hashing again (NULL: hashes).
+ * Everything else as in the calls above. */
+size_t prism_dropout_mask_bytes(int M, int N, int K, int group_size);
+int prism_bwd_dadr_mask(const void* dC, const void* A, const void* B, const void* R, const void* internal_bias,
+                        void* dA, void* dR, void* d_internal_bias, int M, int N, int K, int group_size, int reconn_sz,
+                        int dtype, int gate, int dr_dtype, float dc_scale, long long lddc, long long lda, long long ldb,
+                        long long ldr, long long ldda, long long lddr, const long long* dropout_seeds, float dropout_p,
+                        void* dropout_mask, const int* cfg, void* workspace, size_t workspace_bytes, void* stream);
+int prism_bwd_db_mask(const void* dC, const void* A, const void* R, const void* internal_bias, void* dB,
+                      int M, int N, int K, int group_size, int reconn_sz, int dtype, int gate,
+                      int db_dtype, float dc_scale, long long lddc, long long lda, long long ldr, long long lddb,
+                      const long long* dropout_seeds, float dropout_p, const void* dropout_mask,
+                      const int* cfg, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Output-bias gradient dbias [N] = sum over the M token rows of dC [M,N] (not scaled: the bias is
  * added after the point where the reference's constant backward rescale applies).  The reference adds
  * the bias as a separate torch op (src/cute_prism/_module.py:736-737), whose autograd is this column

@@ -92,3 +92,25 @@ def test_shuffle_copies_are_the_index_operations(G, K, rows, dt):
     out.backward(D64.to(DEV))
     ref.backward(D64)
     assert torch.equal(r_gpu.grad.cpu(), r_cpu.grad)
+
+
+@pytest.mark.parametrize("M,K,p", [(1, 64, 0.5), (130, 200, 0.1), (300, 1096, 2.0 ** -24), (257, 136, 0.999)])
+@pytest.mark.parametrize("ib", [False, True])
+def test_dropout_mask_of_the_dadr_kernel(M, K, p, ib):
+    """dB with the mask that the dA+dR kernel leaves equals dB that hashes for itself, bit for bit, and the oracle."""
+    from cute_mma_b200 import _functional as F
+    N, gs, rs, dt, act = 192, 64, 8, torch.bfloat16, "silu_gate"
+    A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 11)
+    bias = torch.randn(N // gs, K, device=DEV).to(dt) if ib else None
+    seeds = torch.randint(1, 1 << 62, (N // gs,), dtype=torch.int64, device=DEV)
+    dA, dR, dB, _ = cp.backward(dC, A, B, R, gs, rs, activation=act, internal_bias=bias, dropout_seeds=seeds, dropout_p=p)
+    own = F._backward_db(dC, A, R, gs, rs, 1, internal_bias=bias, dropout_seeds=seeds, dropout_p=p)
+    cp.check_device_status()
+    assert torch.equal(dB, own)
+    f = [t.float() for t in (A, B, R)]
+    kw = dict(internal_bias=None if bias is None else bias.float(), dropout_seeds=seeds, dropout_p=p)
+    ref = O.prism_backward(dC.float(), *f, gs, rs, act, **kw)
+    C, _ = cp.forward(A, B, R, gs, rs, activation=act, internal_bias=bias, dropout_seeds=seeds, dropout_p=p, training=True)
+    assert O.rel_err(C.float(), O.prism_forward(*f, gs, rs, act, **kw)) < TOL
+    for got, r in zip((dA, dR, dB), ref):
+        assert O.rel_err(got.float(), r) < TOL
