@@ -275,7 +275,8 @@ extern "C" size_t prism_workspace_bytes(int kind, int M, int N, int K, int gs, i
     const int E = effective_block(rs);
     if (E == 0) return bytes;
     DadrGrid gr;
-    dadr_plan_grid(M, K, num_sms(), cfg, &gr);
+    dadr_plan_grid(M, K, (int)G, gs, num_sms(), cfg, &gr);
+    if (gr.parts > 1) bytes += align256((size_t)gr.parts * M * K * 4);   // fp32 sums for dA of the group parts
     bytes += align256((size_t)2 * gr.runs * G * E * (size_t)K * 4);                 // one buffer per CTA of every main pair
     bytes += align256((size_t)2 * gr.n_extra * gr.slots * G * E * (size_t)128 * 4); // slabs of the extra pairs' CTAs
     if (kind == PRISM_KIND_BWD_DADR_IB) {   // the same for the column sums of dS (gradient of the internal bias)
@@ -486,7 +487,9 @@ extern "C" int prism_bwd_dadr_mask(const void* dC, const void* A, const void* B,
   }
   wp += align256((size_t)(N / gs) * a.E * K * 2);
   a.num_sms = num_sms();
-  dadr_plan_grid(M, K, a.num_sms, cfg, &a.grid);
+  dadr_plan_grid(M, K, N / gs, gs, a.num_sms, cfg, &a.grid);
+  a.partial_da = reinterpret_cast<float*>(wp);
+  if (a.grid.parts > 1) wp += align256((size_t)a.grid.parts * M * K * 4);
   a.partial = reinterpret_cast<float*>(wp);
   wp += align256((size_t)2 * a.grid.runs * (N / gs) * a.E * (size_t)K * 4);
   a.partial_x = reinterpret_cast<float*>(wp);

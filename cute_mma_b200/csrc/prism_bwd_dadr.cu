@@ -73,12 +73,48 @@ __global__ void dib_reduce_kernel(const float* __restrict__ partial, const float
   d_ib[(long long)g * ldib + k] = (uint16_t)(Elem<DT>::pack(acc * scale, 0.f) & 0xffffu);
 }
 
+// dA[m, k] = cast( scale * sum over the group parts of partial[part][m][k] ), in part order; four elements per thread
+// (K is a multiple of 8).
+template <int DT>
+__global__ void __launch_bounds__(256) da_reduce_kernel(const float4* __restrict__ partial, uint16_t* __restrict__ dA, int M,
+                                                        int K, long long ldda, int parts, float scale) {
+  const int m = blockIdx.x;
+  const long long step = (long long)M * (K >> 2);
+  for (int c = threadIdx.x; c < (K >> 2); c += blockDim.x) {
+    const float4* src = partial + (long long)m * (K >> 2) + c;
+    float4 a = __ldg(src);
+    for (int s = 1; s < parts; ++s) {
+      const float4 v = __ldg(src + s * step);
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    *reinterpret_cast<uint2*>(dA + (long long)m * ldda + 4 * c) =
+        make_uint2(Elem<DT>::pack(a.x * scale, a.y * scale), Elem<DT>::pack(a.z * scale, a.w * scale));
+  }
+}
+
+// Groups per part when the tiles alone leave at least half of the SM pairs idle and the groups are split over
+// blockIdx.y (see DadrExtra); G: one part.  A part costs its share of the group steps (about 0.6 us per 64 outputs)
+// plus a pair's start and epilogue; splitting costs the second launch (3 us) and the fp32 sums of dA, written
+// and read once (about 5 TB/s).  Split only for a gain of 2 us or more.
+static int dadr_groups_per_part(int M, int K, int G, int gs, int pairs, int slots) {
+  if (G < 2 || 2 * pairs > slots) return G;
+  const double step = 0.6 * ((gs + 63) / 64);
+  double best_cost = G * step - 2.0;
+  int best = G;
+  for (int parts = 2; parts <= G && pairs * parts <= slots; ++parts) {
+    const int per = (G + parts - 1) / parts;
+    const double cost = per * step + 3.0 + (double)parts * M * K * 8.0 / 5e6;
+    if (cost < best_cost) { best_cost = cost; best = per; }
+  }
+  return best;
+}
+
 // Grid of the dA+dR kernel.  runs: the number of main CTA pairs that share one feature column (each
 // walks every runs-th 256-token tile).  When the main pairs leave SM pairs idle and have enough
 // tiles each, the idle pairs become extra pairs and every main pair leaves its last `steal` tiles
 // to them (see DadrUnit): measured faster than many short runs, with a quarter of the workspace.
 // cfg (or null): {runs, steal, n_extra}; 0 = default; steal < 0 = no extra pairs.
-void dadr_plan_grid(int M, int K, int num_sms, const int* cfg, DadrGrid* gr) {
+void dadr_plan_grid(int M, int K, int G, int gs, int num_sms, const int* cfg, DadrGrid* gr) {
   const int n_ft = (K + 127) / 128;
   const int n_mp = (M + 255) / 256;
   const int slots_sm = num_sms / 2 > 0 ? num_sms / 2 : 1;
@@ -109,6 +145,12 @@ void dadr_plan_grid(int M, int K, int num_sms, const int* cfg, DadrGrid* gr) {
   gr->n_ft = n_ft;
   gr->n_main = n_ft * runs;
   gr->n_extra = 0; gr->steal = 0; gr->slots = 0;
+  gr->g_per = G; gr->parts = 1;
+  if (!cfg || (cfg[0] <= 0 && cfg[1] == 0 && cfg[2] <= 0)) {   // the default plan: no extra pairs beside group parts
+    gr->g_per = dadr_groups_per_part(M, K, G, gs, gr->n_main, slots_sm);
+    gr->parts = (G + gr->g_per - 1) / gr->g_per;
+    if (gr->parts > 1) return;
+  }
   const int t_min = n_mp / runs, t_max = (n_mp + runs - 1) / runs;   // tiles of the shortest / longest run
   int steal = cfg ? cfg[1] : 0;
   int n_extra = (cfg && cfg[2] > 0) ? cfg[2] : (slots_sm - gr->n_main);
@@ -153,6 +195,7 @@ int launch_bwd_dadr(const DadrArgs& a) {
   int smem_bytes = 0;
   const bool ib = a.ib != nullptr && a.gate != GATE_NONE;
   DadrExtra x;
+  x.g_per = a.grid.g_per; x.partial_da = a.partial_da;
   x.ib = ib ? a.ib : nullptr; x.partial_ib = a.partial_ib; x.partial_ib_x = a.partial_ib_x;
   int rc = (a.E == 16) ? dadr_plan<16>(p, smem_bytes, ib) : (a.E == 32) ? dadr_plan<32>(p, smem_bytes, ib) : dadr_plan<64>(p, smem_bytes, ib);
   if (rc) return rc;
@@ -168,11 +211,20 @@ int launch_bwd_dadr(const DadrArgs& a) {
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "bwd_dadr: dropout needs reconn_sz 8 or 16");
   x.drop_seeds = a.drop_seeds; x.drop_thr = drop_threshold(a.drop_p); x.drop_mask = a.drop_mask; x.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
-  DadrKernel kern = (a.dtype == DT_BF16) ? dadr_kernel_bf16(a.gate, a.E, ib, drop) : dadr_kernel_f16(a.gate, a.E, ib, drop);
+  DadrKernel kern = (a.dtype == DT_BF16) ? dadr_kernel_bf16(a.gate, a.E, ib, drop, a.grid.parts > 1)
+                                         : dadr_kernel_f16(a.gate, a.E, ib, drop, a.grid.parts > 1);
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_dadr"))) return rc;
-  dim3 grid(2 * (p.n_main + p.n_extra), 1, 1);   // the two CTAs of a pair are neighbours
+  dim3 grid(2 * (p.n_main + p.n_extra), a.grid.parts, 1);   // the two CTAs of a pair are neighbours
   kern<<<grid, dadr::kThreads, smem_bytes, a.stream>>>(tmA, tmRr, tmRd, tmdC, tmB, p, x);
   if ((rc = check_launch("prism_bwd_dadr"))) return rc;
+  if (a.grid.parts > 1) {
+    const int t = a.K >= 1024 ? 256 : ((a.K >> 2) + 31) / 32 * 32;
+    const float4* src = reinterpret_cast<const float4*>(a.partial_da);
+    uint16_t* dst = reinterpret_cast<uint16_t*>(a.dA);
+    if (a.dtype == DT_BF16) da_reduce_kernel<DT_BF16><<<a.M, t, 0, a.stream>>>(src, dst, a.M, a.K, a.ldda, a.grid.parts, a.scale);
+    else da_reduce_kernel<DT_F16><<<a.M, t, 0, a.stream>>>(src, dst, a.M, a.K, a.ldda, a.grid.parts, a.scale);
+    if ((rc = check_launch("prism_bwd_dadr dA reduce"))) return rc;
+  }
 
   // gated mode: the kernel formed 2 dS against the halved R tiles, so the dR partials are doubled
   const float r_scale = (a.gate != GATE_NONE) ? 0.5f * a.scale : a.scale;

@@ -82,6 +82,10 @@ struct DadrParams {
 // Arguments of the internal-bias and dropout instances only.  A kernel parameter of its own: with these
 // fields inside DadrParams the instance without either (the benchmarked one) compiled to more spills.
 struct DadrExtra {
+  // Few tiles (see dadr_groups_per_part): blockIdx.y splits the groups.  Part y walks groups [y g_per, (y + 1) g_per) and
+  // leaves fp32 sums for dA in partial_da [parts][M][K], which da_reduce_kernel adds; the parts' dR rows are disjoint.
+  int g_per;           // groups per part (all of them: one part, dA written directly)
+  float* partial_da;
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
   uint32_t drop_thr;   // see drop_threshold
   float drop_inv_keep;
@@ -238,7 +242,10 @@ __device__ __forceinline__ float* dadr_unit_ib(const DadrParams& p, const DadrEx
 // sums its 16 token rows with shuffles, the 8 warps of a 64-feature chunk meet in shared memory, are
 // added in a fixed order, and one thread per column stores (first tile) or adds (later tiles).
 // DROP: hash dropout (see drop_mask32): dH is multiplied by the forward's mask before it is used.
-template <int DT, int GATE, int E, bool IB, bool DROP>
+// PARTS: the groups may be split over blockIdx.y (see DadrExtra).  The instances that can be split run 3 % (fp16) and 1.5 %
+// (plain mode) slower on one part than those that cannot, so both exist; with bf16 gates it is the other way round (fewer
+// spills: 16384 x 4096 -> 14336 4.22 -> 4.00 ms, 8192 x 1024 -> 16384 560 -> 540 us) and there is only the former.
+template <int DT, int GATE, int E, bool IB, bool DROP, bool PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(dadr::kThreads, 1)
 prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmRr,
                       const __grid_constant__ CUtensorMap tmRd, const __grid_constant__ CUtensorMap tmdC,
@@ -266,7 +273,9 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();   // 0 = leader (issues the MMAs), 1 = peer
   const int pidx = blockIdx.x >> 1;          // CTA pair: main pairs first, then the extra pairs
-  const int G = p.G;
+  const int g_lo = PARTS ? blockIdx.y * ex.g_per : 0;
+  const int g_hi = PARTS ? min(p.G, g_lo + ex.g_per) : p.G;   // this part's groups: [g_lo, g_hi) ...
+  const int G = PARTS ? g_hi - g_lo : p.G;                    // ... and their count
   const int nstg = (p.gs + St::kOut - 1) / St::kOut;  // stages per group
   const bool is_gate = warp >= kGateWarp0 && warp < kGateWarp0 + kNumGateWarps;
   const bool is_dr = warp == 2 || warp == 3 || warp == 20 || warp == 21;
@@ -327,7 +336,7 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         mbar_arrive_expect_tx(&bars->a_full, 2 * kTile);
         tma_load_2d(smemA, &tmA, &bars->a_full, f0, m0);
         tma_load_2d(smemA + kTile, &tmA, &bars->a_full, f0 + 64, m0);
-        for (int g = 0; g < G && ok; ++g, rr.next()) {
+        for (int g = g_lo; g < g_hi && ok; ++g, rr.next()) {
           if (!mbar_wait(&bars->r_empty[rr.idx], rr.phase ^ 1)) { ok = false; break; }
           uint8_t* dstR = smemR + rr.idx * r_buf_bytes;
           const uint32_t rfull = mapa_shared(smem_u32(&bars->r_full[rr.idx]), 0);
@@ -530,7 +539,7 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         ib_valid = p.K - (f0 + ch * 64);
       }
       if (!mbar_wait(&bars->a_full, tile_iter & 1)) { ok = false; break; }
-      for (int g = 0; g < G && ok; ++g, ++gg) {
+      for (int g = g_lo; g < g_hi && ok; ++g, ++gg) {
         const uint32_t hb = gg & 1, ph = (gg >> 1) & 1;
         uint32_t mask = 0;
         if (DROP && kGated) {   // before the waits: the hash needs indices only
@@ -677,6 +686,7 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       tc_fence_after_sync();
       const long long grow = (long long)mt * 128 + r0 + (lane >> 2);
       uint16_t* out = reinterpret_cast<uint16_t*>(p.dA);
+      float* out32 = PARTS && gridDim.y > 1 ? ex.partial_da + (long long)blockIdx.y * p.M * p.K : nullptr;
 #pragma unroll
       for (int pc = 0; pc < 4; ++pc) {
         uint32_t v[8];
@@ -686,7 +696,14 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         for (int hh = 0; hh < 2; ++hh) {   // columns 0-7 / 8-15 of the piece
           const int nt = pc * 2 + hh;
           const int col = f0 + ch * 64 + nt * 8 + (lane & 3) * 2;
-          if (col < p.K) {
+          if (PARTS && col < p.K && out32 != nullptr) {
+            if (grow < p.M)
+              *reinterpret_cast<float2*>(out32 + grow * p.K + col) =
+                  make_float2(dacc[nt][0] + __uint_as_float(v[hh * 4 + 0]), dacc[nt][1] + __uint_as_float(v[hh * 4 + 1]));
+            if (grow + 8 < p.M)
+              *reinterpret_cast<float2*>(out32 + (grow + 8) * p.K + col) =
+                  make_float2(dacc[nt][2] + __uint_as_float(v[hh * 4 + 2]), dacc[nt][3] + __uint_as_float(v[hh * 4 + 3]));
+          } else if (col < p.K) {
             if (grow < p.M)
               *reinterpret_cast<uint32_t*>(out + grow * p.ldda + col) =
                   Elem<DT>::pack((dacc[nt][0] + __uint_as_float(v[hh * 4 + 0])) * p.scale,
@@ -715,7 +732,7 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const int f0 = tu.f0;
       const bool first = tu.first;
       if (!mbar_wait(&bars->a_full, tile_iter & 1)) { ok = false; break; }
-      for (int g = 0; g < G && ok; ++g, ++gg) {
+      for (int g = g_lo; g < g_hi && ok; ++g, ++gg) {
         const int buf = gg & 1;
         if (!mbar_wait(&bars->ds_full[buf], (gg >> 1) & 1)) { ok = false; break; }
         for (int u = w; u < n_sub; u += kNumDrWarps) {
@@ -789,19 +806,24 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 }
 
 using DadrKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, DadrParams, DadrExtra);
-// kernel instance for (gate, E, internal-bias variant), one function per data type and translation unit
-DadrKernel dadr_kernel_f16(int gate, int E, bool ib, bool drop);
-DadrKernel dadr_kernel_bf16(int gate, int E, bool ib, bool drop);
+// kernel instance for (gate, E, internal-bias variant, dropout, groups split into parts), one function per data type and
+// translation unit
+DadrKernel dadr_kernel_f16(int gate, int E, bool ib, bool drop, bool parts);
+DadrKernel dadr_kernel_bf16(int gate, int E, bool ib, bool drop, bool parts);
 
+#define PRISM_DADR_PICK_P(DT_, G_, E_, IB_, DROP_)                                                           \
+  (parts || (DT_ == DT_BF16 && G_ != GATE_NONE)                                                              \
+       ? (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, IB_, DROP_, true>                                     \
+       : (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, IB_, DROP_, (DT_ == DT_BF16 && G_ != GATE_NONE)>)
 #define PRISM_DADR_PICK_IB(DT_, G_, E_, DROP_) \
-  (ib ? (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, true, DROP_> : (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, false, DROP_>)
+  (ib ? PRISM_DADR_PICK_P(DT_, G_, E_, true, DROP_) : PRISM_DADR_PICK_P(DT_, G_, E_, false, DROP_))
 #define PRISM_DADR_PICK_G(DT_, E_, DROP_)                                                        \
   (gate == GATE_SILU ? PRISM_DADR_PICK_IB(DT_, GATE_SILU, E_, DROP_)                              \
    : gate == GATE_SIGMOID ? PRISM_DADR_PICK_IB(DT_, GATE_SIGMOID, E_, DROP_)                      \
-                          : (DadrKernel)prism_bwd_dadr_kernel<DT_, GATE_NONE, E_, false, false>)
+                          : PRISM_DADR_PICK_P(DT_, GATE_NONE, E_, false, false))
 // dropout kernels exist for E = 16 (reconn_sz 8 and 16) only
 #define PRISM_DADR_DEFINE_PICKER(NAME_, DT_)                                  \
-  DadrKernel NAME_(int gate, int E, bool ib, bool drop) {                     \
+  DadrKernel NAME_(int gate, int E, bool ib, bool drop, bool parts) {         \
     if (drop) return PRISM_DADR_PICK_G(DT_, 16, true);                        \
     if (E == 16) return PRISM_DADR_PICK_G(DT_, 16, false);                    \
     if (E == 32) return PRISM_DADR_PICK_G(DT_, 32, false);                    \

@@ -80,6 +80,8 @@ struct DadrGrid {
   int n_extra;   // extra CTA pairs that take over the main pairs' last tiles (0: none)
   int steal;     // tiles every main pair leaves to them
   int slots;     // dR slabs per extra CTA
+  int g_per;     // groups per part ...
+  int parts;     // ... and parts (blockIdx.y): 1, or few tiles with the groups split over the idle SM pairs
 };
 struct DadrArgs {
   const void* dC;     // [M, N]
@@ -103,11 +105,12 @@ struct DadrArgs {
   DadrGrid grid;      // CTA pairs and their tiles
   float* partial;     // [2*runs][(N/gs)*E][K] fp32: dR buffers of the main pairs' CTAs
   float* partial_x;   // [2*n_extra][slots][(N/gs)*E][128] fp32: dR slabs of the extra pairs' CTAs
+  float* partial_da;  // [parts][M][K] fp32: sums for dA, when the groups are split into parts
   int num_sms;
   int* err;
   cudaStream_t stream;
 };
 int launch_bwd_dadr(const DadrArgs& a);
-void dadr_plan_grid(int M, int K, int num_sms, const int* cfg, DadrGrid* grid);
+void dadr_plan_grid(int M, int K, int G, int gs, int num_sms, const int* cfg, DadrGrid* grid);
 
 }  // namespace prism

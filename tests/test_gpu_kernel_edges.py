@@ -114,3 +114,29 @@ def test_dropout_mask_of_the_dadr_kernel(M, K, p, ib):
     assert O.rel_err(C.float(), O.prism_forward(*f, gs, rs, act, **kw)) < TOL
     for got, r in zip((dA, dR, dB), ref):
         assert O.rel_err(got.float(), r) < TOL
+
+
+@pytest.mark.parametrize("M,K,G,gs", [(1, 64, 12, 96), (100, 72, 9, 96), (300, 520, 7, 128), (1000, 264, 3, 512)])
+@pytest.mark.parametrize("opts", ["plain", "gate", "ib", "drop"])
+def test_group_parts_of_dadr(M, K, G, gs, opts):
+    """Few tiles: the groups split over CTA pairs against one part (a plan given by hand is never split) and the oracle.
+    A group's dR does not depend on the split; dA's partial sums meet in fp32."""
+    from cute_mma_b200 import _functional as F
+    from cute_mma_b200 import _lib
+    N, rs, dt = G * gs, 8, torch.bfloat16
+    act, gate = (None, 0) if opts == "plain" else ("silu_gate", 1)
+    A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 13)
+    ib = torch.randn(G, K, device=DEV).to(dt) if opts == "ib" else None
+    kw = dict(dropout_seeds=torch.arange(1, G + 1, device=DEV), dropout_p=0.25) if opts == "drop" else {}
+    before = _lib.lib().prism_launch_count()
+    got = F._backward_dadr(dC, A, B, R, gs, rs, gate, internal_bias=ib, **kw)
+    n_split = _lib.lib().prism_launch_count() - before
+    one = F._backward_dadr(dC, A, B, R, gs, rs, gate, internal_bias=ib, tile_cfg=[0, -1, 0], **kw)
+    n_one = _lib.lib().prism_launch_count() - before - n_split
+    cp.check_device_status()
+    assert n_split == n_one + 1, "this shape is meant to be split"
+    ref = O.prism_backward(dC.float(), A.float(), B.float(), R.float(), gs, rs, act,
+                           internal_bias=None if ib is None else ib.float(), **kw)
+    assert torch.equal(got[1], one[1]) and (ib is None or torch.equal(got[2], one[2]))
+    assert O.rel_err(got[0].float(), one[0].float()) < 2 ** -8 + 1e-3    # one rounding to bf16 on either side
+    assert O.rel_err(got[0].float(), ref[0]) < TOL and O.rel_err(got[1].float(), ref[1]) < TOL
