@@ -90,8 +90,7 @@ class _WorkspacePool:
         self._retired = []   # [(device, tensor)] replaced by a larger buffer, status not read yet
 
     def get(self, device: torch.device, nbytes: int) -> torch.Tensor:
-        stream = torch.cuda.current_stream(device)
-        key = (device, stream.cuda_stream)
+        key = (device, _raw_stream(device))
         with self._lock:
             buf = self._bufs.get(key)
             if buf is None or buf.numel() < nbytes:
@@ -123,7 +122,7 @@ _workspace = _WorkspacePool()
 def _read_status(device, buf) -> None:
     with torch.cuda.device(device):
         torch.cuda.synchronize(device)
-        _lib.check(_lib.lib().prism_status(ctypes.c_void_p(buf.data_ptr()), _stream_ptr(device)))
+        _lib.check(_lib.lib().prism_status(ctypes.c_void_p(buf.data_ptr()), _raw_stream(device)))
 
 
 def _cfg_array(cfg):
@@ -133,8 +132,39 @@ def _cfg_array(cfg):
     return arr
 
 
-def _stream_ptr(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _raw_stream(device) -> int:
+    """The device's current CUDA stream as a handle, without a Stream object."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+class _NoScope:
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_no_scope = _NoScope()
+
+
+def _device_scope(device):
+    """The device made current for a launch; nothing to do (and nothing to pay) where it already is."""
+    return _no_scope if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+_need_cache: dict = {}
+
+
+def _workspace_need(L, kind, M, N, K, group_size, reconn_sz, dt, cfg, cfg_arr, device) -> int:
+    """``prism_workspace_bytes``, a function of these arguments alone, remembered for the latest calls."""
+    key = (kind, M, N, K, group_size, reconn_sz, dt, None if cfg is None else tuple(cfg), device.index)
+    need = _need_cache.get(key)
+    if need is None:
+        if len(_need_cache) >= 512:
+            _need_cache.clear()
+        need = _need_cache[key] = L.prism_workspace_bytes(kind, M, N, K, group_size, reconn_sz, dt, cfg_arr)
+    return need
 
 
 def check_device_status(device=None) -> None:
@@ -194,7 +224,7 @@ def _check_seeds(seeds, A, n_groups):
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _reject_unsupported(**kw):
@@ -278,15 +308,15 @@ def forward(A, B, R, group_size: int = 256, reconn_sz: int = 8, backend=None, mo
     cfg = tile_cfg if tile_cfg is not None else _tile_lookup("fwd", A.dtype, gate, M, N, K, group_size, reconn_sz)
     cfg_arr = _cfg_array(cfg)
     dt = _DTYPES[A.dtype]
-    with torch.cuda.device(A.device):
-        need = L.prism_workspace_bytes(KIND_FWD, M, N, K, group_size, reconn_sz, dt, cfg_arr)
+    with _device_scope(A.device):
+        need = _workspace_need(L, KIND_FWD, M, N, K, group_size, reconn_sz, dt, cfg, cfg_arr, A.device)
         ws = _workspace.get(A.device, need)
         _lib.check(L.prism_fwd_dropout(
-            ctypes.c_void_p(A.data_ptr()), ctypes.c_void_p(B.data_ptr()), ctypes.c_void_p(R.data_ptr()),
-            _ptr(bias), _ptr(internal_bias), ctypes.c_void_p(C.data_ptr()),
+            A.data_ptr(), B.data_ptr(), R.data_ptr(),
+            _ptr(bias), _ptr(internal_bias), C.data_ptr(),
             M, N, K, group_size, reconn_sz, dt, gate, A.stride(0), B.stride(0), R.stride(0), C.stride(0),
-            _ptr(seeds), ctypes.c_float(dropout_p if seeds is not None else 0.0),
-            cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
+            _ptr(seeds), dropout_p if seeds is not None else 0.0,
+            cfg_arr, ws.data_ptr(), ws.numel(), _raw_stream(A.device)))
     return C, ([seeds] if seeds is not None else [])
 
 
@@ -306,10 +336,10 @@ def fold_weight(B, R, group_size: int, reconn_sz: int):
     validate_kernel_params(group_size, reconn_sz)
     N, K = B.shape
     Bp = torch.empty_like(B)
-    with torch.cuda.device(B.device):
+    with _device_scope(B.device):
         _lib.check(_lib.lib().prism_fold_weight(
-            ctypes.c_void_p(B.data_ptr()), ctypes.c_void_p(R.data_ptr()), ctypes.c_void_p(Bp.data_ptr()),
-            N, K, group_size, reconn_sz, _DTYPES[B.dtype], B.stride(0), R.stride(0), Bp.stride(0), _stream_ptr(B.device)))
+            B.data_ptr(), R.data_ptr(), Bp.data_ptr(),
+            N, K, group_size, reconn_sz, _DTYPES[B.dtype], B.stride(0), R.stride(0), Bp.stride(0), _raw_stream(B.device)))
     return Bp
 
 
@@ -325,10 +355,10 @@ def cayley(M, reconn_sz: int):
     ``S = M - M^T``, ``R = (I - S)^-1 (I + S)`` through ``prism_cayley`` (fp32 inside)."""
     M = M.contiguous()
     R = torch.empty_like(M)
-    with torch.cuda.device(M.device):
-        _lib.check(_lib.lib().prism_cayley(ctypes.c_void_p(M.data_ptr()), ctypes.c_void_p(R.data_ptr()),
+    with _device_scope(M.device):
+        _lib.check(_lib.lib().prism_cayley(M.data_ptr(), R.data_ptr(),
                                            M.shape[0] // reconn_sz, M.shape[1], reconn_sz, _CAYLEY_DTYPES[M.dtype],
-                                           M.stride(0), R.stride(0), _stream_ptr(M.device)))
+                                           M.stride(0), R.stride(0), _raw_stream(M.device)))
     return R
 
 
@@ -336,11 +366,11 @@ def cayley_backward(M, dR, reconn_sz: int):
     """Gradient of ``cayley`` with respect to ``M`` through ``prism_cayley_bwd``."""
     M, dR = M.contiguous(), dR.contiguous().to(M.dtype)
     dM = torch.empty_like(M)
-    with torch.cuda.device(M.device):
-        _lib.check(_lib.lib().prism_cayley_bwd(ctypes.c_void_p(M.data_ptr()), ctypes.c_void_p(dR.data_ptr()),
-                                               ctypes.c_void_p(dM.data_ptr()), M.shape[0] // reconn_sz, M.shape[1], reconn_sz,
+    with _device_scope(M.device):
+        _lib.check(_lib.lib().prism_cayley_bwd(M.data_ptr(), dR.data_ptr(),
+                                               dM.data_ptr(), M.shape[0] // reconn_sz, M.shape[1], reconn_sz,
                                                _CAYLEY_DTYPES[M.dtype], M.stride(0), dR.stride(0), dM.stride(0),
-                                               _stream_ptr(M.device)))
+                                               _raw_stream(M.device)))
     return dM
 
 
@@ -356,9 +386,9 @@ def shuffle_cols(X, seg):
     X = _segment_aligned(X)
     G, K = seg.shape[0], seg.shape[1] * 64
     Y = torch.empty_like(X)
-    with torch.cuda.device(X.device):
+    with _device_scope(X.device):
         _lib.check(_lib.lib().prism_shuffle_cols(_ptr(X), _ptr(Y), _ptr(seg), G, X.shape[0] // G, K, X.element_size(),
-                                                 _stream_ptr(X.device)))
+                                                 _raw_stream(X.device)))
     return Y
 
 
@@ -367,8 +397,8 @@ def shuffle_fold_r(R, inv_seg):
     R = _segment_aligned(R)
     G, K = inv_seg.shape[0], inv_seg.shape[1] * 64
     R64 = torch.empty(G * 64, K, dtype=R.dtype, device=R.device)
-    with torch.cuda.device(R.device):
-        _lib.check(_lib.lib().prism_shuffle_fold_r(_ptr(R), _ptr(R64), _ptr(inv_seg), G, K, _stream_ptr(R.device)))
+    with _device_scope(R.device):
+        _lib.check(_lib.lib().prism_shuffle_fold_r(_ptr(R), _ptr(R64), _ptr(inv_seg), G, K, _raw_stream(R.device)))
     return R64
 
 
@@ -377,9 +407,9 @@ def shuffle_unfold_r(dR64, perm_seg):
     dR64 = _segment_aligned(dR64)
     G, K = perm_seg.shape[0], perm_seg.shape[1] * 64
     dR = torch.empty(G * 16, K, dtype=dR64.dtype, device=dR64.device)
-    with torch.cuda.device(dR.device):
+    with _device_scope(dR.device):
         _lib.check(_lib.lib().prism_shuffle_unfold_r(_ptr(dR64), _ptr(dR), _ptr(perm_seg), G, K, dR64.element_size(),
-                                                     _stream_ptr(dR.device)))
+                                                     _raw_stream(dR.device)))
     return dR
 
 
@@ -416,14 +446,14 @@ def _backward_db(dC, A, R, group_size, reconn_sz, gate, dc_scale=1.0, tile_cfg=N
     cfg = tile_cfg if tile_cfg is not None else _tile_lookup("bwd_db", A.dtype, gate, M, N, K, group_size, reconn_sz)
     cfg_arr = _cfg_array(cfg)
     dt = _DTYPES[A.dtype]
-    with torch.cuda.device(A.device):
-        need = L.prism_workspace_bytes(KIND_BWD_DB, M, N, K, group_size, reconn_sz, dt, cfg_arr)
+    with _device_scope(A.device):
+        need = _workspace_need(L, KIND_BWD_DB, M, N, K, group_size, reconn_sz, dt, cfg, cfg_arr, A.device)
         ws = _workspace.get(A.device, need)
         _lib.check(L.prism_bwd_db_mask(
-            ctypes.c_void_p(dC.data_ptr()), ctypes.c_void_p(A.data_ptr()), ctypes.c_void_p(R.data_ptr()),
-            _ptr(internal_bias), ctypes.c_void_p(dB.data_ptr()), M, N, K, group_size, reconn_sz, dt, gate, out_code,
-            ctypes.c_float(dc_scale), dC.stride(0), A.stride(0), R.stride(0), dB.stride(0),
-            _ptr(dropout_seeds), ctypes.c_float(dropout_p if dropout_seeds is not None else 0.0), _ptr(dropout_mask), cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
+            dC.data_ptr(), A.data_ptr(), R.data_ptr(),
+            _ptr(internal_bias), dB.data_ptr(), M, N, K, group_size, reconn_sz, dt, gate, out_code,
+            dc_scale, dC.stride(0), A.stride(0), R.stride(0), dB.stride(0),
+            _ptr(dropout_seeds), dropout_p if dropout_seeds is not None else 0.0, _ptr(dropout_mask), cfg_arr, ws.data_ptr(), ws.numel(), _raw_stream(A.device)))
     return dB
 
 
@@ -442,17 +472,17 @@ def _backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, dc_scale=1.0, tile_
     cfg = tile_cfg if tile_cfg is not None else _tile_lookup("bwd_dadr", A.dtype, gate, M, N, K, group_size, reconn_sz)
     cfg_arr = _cfg_array(cfg)
     dt = _DTYPES[A.dtype]
-    with torch.cuda.device(A.device):
+    with _device_scope(A.device):
         kind = KIND_BWD_DADR_IB if internal_bias is not None else KIND_BWD_DADR
-        need = L.prism_workspace_bytes(kind, M, N, K, group_size, reconn_sz, dt, cfg_arr)
+        need = _workspace_need(L, kind, M, N, K, group_size, reconn_sz, dt, cfg, cfg_arr, A.device)
         ws = _workspace.get(A.device, need)
         _lib.check(L.prism_bwd_dadr_mask(
-            ctypes.c_void_p(dC.data_ptr()), ctypes.c_void_p(A.data_ptr()), ctypes.c_void_p(B.data_ptr()),
-            ctypes.c_void_p(R.data_ptr()), _ptr(internal_bias), ctypes.c_void_p(dA.data_ptr()),
-            ctypes.c_void_p(dR.data_ptr()), _ptr(d_ib),
-            M, N, K, group_size, reconn_sz, dt, gate, dr_code, ctypes.c_float(dc_scale),
+            dC.data_ptr(), A.data_ptr(), B.data_ptr(),
+            R.data_ptr(), _ptr(internal_bias), dA.data_ptr(),
+            dR.data_ptr(), _ptr(d_ib),
+            M, N, K, group_size, reconn_sz, dt, gate, dr_code, dc_scale,
             dC.stride(0), A.stride(0), B.stride(0), R.stride(0), dA.stride(0), dR.stride(0),
-            _ptr(dropout_seeds), ctypes.c_float(dropout_p if dropout_seeds is not None else 0.0), _ptr(dropout_mask), cfg_arr, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(A.device)))
+            _ptr(dropout_seeds), dropout_p if dropout_seeds is not None else 0.0, _ptr(dropout_mask), cfg_arr, ws.data_ptr(), ws.numel(), _raw_stream(A.device)))
     if internal_bias is not None:
         return dA, dR, d_ib
     return dA, dR
@@ -515,9 +545,9 @@ def bias_grad(dC, out_dtype=None):
     out = torch.empty(N, dtype=out_dtype, device=dC.device)
     L = _lib.lib()
     dt = _DTYPES[dC.dtype]
-    with torch.cuda.device(dC.device):
-        need = L.prism_workspace_bytes(KIND_DBIAS, M, N, 0, 0, 0, dt, None)
+    with _device_scope(dC.device):
+        need = _workspace_need(L, KIND_DBIAS, M, N, 0, 0, 0, dt, None, None, dC.device)
         ws = _workspace.get(dC.device, need)
-        _lib.check(L.prism_dbias(ctypes.c_void_p(dC.data_ptr()), ctypes.c_void_p(out.data_ptr()), M, N, dt, out_code,
-                                 dC.stride(0), ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(dC.device)))
+        _lib.check(L.prism_dbias(dC.data_ptr(), out.data_ptr(), M, N, dt, out_code,
+                                 dC.stride(0), ws.data_ptr(), ws.numel(), _raw_stream(dC.device)))
     return out

@@ -207,11 +207,97 @@ def _backward(ctx, dC):
 _prism_forward_op.register_autograd(_backward, setup_context=_setup_context)
 
 
+# ---------------------------------------------------------------------------
+# the eager path: one autograd node for the whole layer
+# ---------------------------------------------------------------------------
+def _plain_eager(*tensors) -> bool:
+    """Whether this call is ordinary eager work on CUDA tensors.  Tracing, compilation, dispatch and function modes, torch.func
+    transforms, forward-mode differentiation and tensor subclasses have to see the custom ops, which describe themselves
+    to all of these; an ordinary call only pays for that (a custom op costs about 50 us of host time in each direction)."""
+    if (torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
+            or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
+            or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0):
+        return False
+    for t in tensors:
+        if t is not None and (type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda):
+            return False
+    return True
+
+
+def _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p, fold, cayley):
+    """(C, and the contiguous tensors the kernels were given): P is R, or the Cayley parameter it is made from."""
+    A, weight, P = A.contiguous(), weight.contiguous(), P.contiguous()
+    R, rs = P, reconn_sz
+    if cayley:
+        R = F.cayley(P, reconn_sz)
+    if fold is not None:
+        weight, R, rs = F.shuffle_cols(weight, fold.inv_seg), F.shuffle_fold_r(R, fold.inv_seg), 64
+        ib = None if ib is None else F.shuffle_cols(ib, fold.inv_seg)
+    C, _ = F.forward(A, weight, R, group_size, rs, activation=activation or None, bias=bias, internal_bias=ib,
+                     dropout_p=dropout_p, training=seeds is not None, dropout_seeds=seeds)
+    return C, A, weight, P, R, ib
+
+
+class _LayerFn(torch.autograd.Function):
+    """The layer as one autograd node, with the gradients that the custom ops return."""
+
+    @staticmethod
+    def forward(ctx, A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, cayley):
+        C, A, weight, P, R, ib = _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p,
+                                                fold, cayley)
+        ctx.save_for_backward(A, weight, R, ib, P if cayley else None)
+        ctx.args = group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, bias is not None, seeds
+        return C
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dC):
+        A, weight, R, ib, P = ctx.saved_tensors
+        group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, has_bias, seeds = ctx.args
+        rs = reconn_sz if fold is None else 64
+        dC = dC.contiguous()
+        gate = F._gate_code(activation or None)
+        ib = None if ib is None else ib.contiguous()
+        need_dB = ctx.needs_input_grad[1]
+        mask = F._dropout_mask(seeds if need_dB and gate else None, A.shape[0], weight.shape[0], A.shape[1], group_size)
+        out = F._backward_dadr(dC, A, weight, R, group_size, rs, gate, bwd_scale, internal_bias=ib,
+                               dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
+        dA, dP = out[0], out[1]
+        d_ib = out[2] if ib is not None else None
+        dB = None
+        if need_dB:
+            if gate:
+                dB = F._backward_db(dC, A, R, group_size, rs, gate, bwd_scale, internal_bias=ib,
+                                    dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
+            else:
+                dB = torch.zeros_like(weight)  # frozen-B contract of the reference's plain mode
+        # the bias is added after the rescale point: its gradient is the plain column sum of dC
+        dbias = F.bias_grad(dC) if has_bias and ctx.needs_input_grad[3] else None
+        if fold is not None:
+            dP = F.shuffle_unfold_r(dP, fold.perm_seg)
+            dB = None if dB is None else F.shuffle_cols(dB, fold.perm_seg)
+            d_ib = None if d_ib is None else F.shuffle_cols(d_ib, fold.perm_seg)
+        if P is not None and ctx.needs_input_grad[2]:
+            dP = F.cayley_backward(P, dP, reconn_sz)
+        return dA, dB, dP, dbias, d_ib, None, None, None, None, None, None, None, None
+
+
+def _layer_eager(A, weight, P, bias, ib, seeds, *args):
+    group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, cayley = args
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (A, weight, P, bias, ib)):
+        return _LayerFn.apply(A, weight, P, bias, ib, seeds, *args)
+    return _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p, fold, cayley)[0]
+
+
 def prism_linear(A, B, R, bias=None, group_size=256, reconn_sz=8, activation=None, bwd_scale=1.0,
                  internal_bias=None, dropout_seeds=None, dropout_p=0.0):
     """Differentiable functional form: C = prism(A, B, R) + bias; gradients of A/B/R (and of the
     internal bias) are multiplied by ``bwd_scale`` (the output-bias gradient is not).  ``dropout_seeds``
     (int64, one per group) switches the hash dropout of the gated activation on."""
+    if _plain_eager(A, B, R, bias, internal_bias, dropout_seeds):
+        return _layer_eager(A, B, R, bias, internal_bias, dropout_seeds, group_size, reconn_sz, activation or "",
+                            float(bwd_scale), float(dropout_p), None, False)
     return _prism_forward_op(A, B, R, bias, group_size, reconn_sz, activation or "", float(bwd_scale), internal_bias,
                              dropout_seeds, float(dropout_p))
 
@@ -370,21 +456,31 @@ class PrismLinear(nn.Module):
         return layer
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        A = input.reshape(-1, self.in_features)
+        A = input if input.dim() == 2 and input.shape[1] == self.in_features else input.reshape(-1, self.in_features)
         seeds = None
         if self.training and self.dropout > 0.0 and self.activation in _GATED:
             # one seed per group and call; forward and backward regenerate the mask from them
             seeds = torch.randint(1, 1 << 62, (self.out_features // self.group_size,), dtype=torch.int64,
                                   device=A.device)
-        weight, R, rs, ib = self.weight, self._build_R(), self.reconn_sz, self._internal_bias
+        weight, P, ib, fold = self.weight, self.reconn, self._internal_bias, None
         if self.input_shuffle:
             # every group's permutation of the input features, folded into the parameters: a 64-wide rotation
-            # on the same kernels (``_shuffle``); autograd carries dR, dB and the bias gradient back through the fold
+            # on the same kernels (``_shuffle``); dR, dB and the bias gradient come back through the fold
             fold = self._shuffle_fold
             if fold is None or fold.perm.device != A.device:
                 from ._shuffle import ShuffleFold
                 fold = self._shuffle_fold = ShuffleFold(self._shuffle_masks, self.in_features, self.group_size,
                                                         self.reconn_sz, A.device)
+        if _plain_eager(A, weight, P, self.ar_scale, self.bias, ib) and (fold is None or (
+                fold._native(weight, self.group_size) and fold._native(P, self.reconn_sz) and self.ar_scale is None
+                and (ib is None or fold._native(ib, 1)))):
+            cayley = (self.activation not in _GATED and self.cayley_order == float("inf")
+                      and F.cayley_supported(P, self.reconn_sz))
+            C = _layer_eager(A, weight, P if cayley else self._build_R(), self.bias, ib, seeds, self.group_size,
+                             self.reconn_sz, self.activation or "", float(self._bwd_scale), self.dropout, fold, cayley)
+            return C if A is input else C.reshape(input.shape[:-1] + (self.out_features,))
+        R, rs = self._build_R(), self.reconn_sz
+        if fold is not None:
             weight, R, rs = fold.fold_cols(weight, self.group_size), fold.fold_R(R), 64
             ib = None if ib is None else fold.fold_cols(ib, 1)
         C = _prism_forward_op(A, weight, R, self.bias, self.group_size, rs,

@@ -15,6 +15,7 @@ import os
 import torch
 
 _TABLE = None
+_FOUND: dict = {}   # answers of the table that is loaded, for the latest calls
 _DT = {torch.float16: "fp16", torch.bfloat16: "bf16"}
 
 
@@ -25,6 +26,7 @@ def table_path() -> str:
 
 def load(path: str | None = None):
     global _TABLE
+    _FOUND.clear()
     path = path or table_path()
     try:
         with open(path) as f:
@@ -41,6 +43,10 @@ def _match(v, want):
 def lookup(kernel, dtype, gate, M, N, K, gs, rs):
     if _TABLE is None:
         load()
+    key = (kernel, dtype, gate, M, N, K, gs, rs)
+    found = _FOUND.get(key, _FOUND)
+    if found is not _FOUND:
+        return None if found is None else list(found)
     best = None
     for e in _TABLE:
         if not (_match(e.get("kernel", "*"), kernel) and _match(e.get("dtype", "*"), _DT.get(dtype, str(dtype)))
@@ -51,4 +57,7 @@ def lookup(kernel, dtype, gate, M, N, K, gs, rs):
         m = 0 if m == "*" else m
         if m <= M and (best is None or m >= best[0]):
             best = (m, e["cfg"])
+    if len(_FOUND) >= 512:
+        _FOUND.clear()
+    _FOUND[key] = None if best is None else tuple(best[1])
     return None if best is None else list(best[1])

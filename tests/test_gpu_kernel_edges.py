@@ -140,3 +140,99 @@ def test_group_parts_of_dadr(M, K, G, gs, opts):
     assert torch.equal(got[1], one[1]) and (ib is None or torch.equal(got[2], one[2]))
     assert O.rel_err(got[0].float(), one[0].float()) < 2 ** -8 + 1e-3    # one rounding to bf16 on either side
     assert O.rel_err(got[0].float(), ref[0]) < TOL and O.rel_err(got[1].float(), ref[1]) < TOL
+
+
+class _Seen(torch.utils._python_dispatch.TorchDispatchMode):
+    """Runs every op as it comes and remembers the package's own."""
+
+    def __init__(self):
+        super().__init__()
+        self.ops = set()
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        if func.namespace == "prism_b200":
+            self.ops.add(func.__name__)
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(bias=False, reconn_sz=16), dict(reconn_sz=32), dict(cayley_order=2),
+                                dict(activation="silu_gate", internal_bias=True), dict(activation="sigmoid_gate", ar_scale_init=0.7),
+                                dict(activation="silu_gate", dropout=0.2, internal_bias=True),
+                                dict(activation="silu_gate", input_shuffle=True, reconn_sz=16, internal_bias=True),
+                                dict(input_shuffle=True, reconn_sz=16)])
+@pytest.mark.parametrize("train_weight", [False, True])
+def test_eager_layer_is_the_custom_ops(kw, train_weight):
+    """An ordinary call runs as one autograd node, a call under a dispatch mode as the custom ops: the same numbers, the
+    same gradients, for a strided 3-D input and a strided output gradient, twice through a retained graph."""
+    from cute_mma_b200 import _module
+    K, N, dt = 192, 256, torch.bfloat16
+    torch.manual_seed(1)
+    layer = cp.PrismLinear(K, N, **{"group_size": 64, "reconn_sz": 8, **kw})
+    if not layer.activation:
+        torch.nn.init.normal_(layer.reconn, 0.0, 0.1)
+    layer = layer.to(DEV).to(dt).train()
+    layer.weight.requires_grad_(train_weight)
+    x0 = torch.randn(5, 2 * K, 34, device=DEV).to(dt)
+    dy = torch.randn(N, 5, 34, device=DEV).to(dt).permute(1, 2, 0)
+    res = []
+    for mode in (None, _Seen()):
+        x = x0[:, ::2].transpose(1, 2).detach().requires_grad_()
+        layer.zero_grad(set_to_none=True)
+        torch.manual_seed(2)   # dropout seeds
+        if mode is None:
+            assert _module._plain_eager(x, layer.weight)
+            y = layer(x)
+            y.backward(dy, retain_graph=True)
+            y.backward(dy)
+        else:
+            with mode:
+                assert not _module._plain_eager(x, layer.weight)
+                y = layer(x)
+                y.backward(dy, retain_graph=True)
+                y.backward(dy)
+            assert "forward.default" in mode.ops
+        res.append([y.detach(), x.grad] + [p.grad for p in layer.parameters()])
+    with torch.no_grad():
+        torch.manual_seed(2)
+        assert torch.equal(layer(x0[:, ::2].transpose(1, 2)), res[0][0])
+    cp.check_device_status()
+    assert (res[0][2] is None) == (not train_weight)
+    for a, b in zip(*res):
+        assert (a is None and b is None) or torch.equal(a, b)
+
+
+def test_eager_layer_under_autograd_features():
+    from cute_mma_b200 import _module
+    K, N, dt = 128, 128, torch.float16
+    layer = cp.PrismLinear(K, N, group_size=64, reconn_sz=8, activation="silu_gate").to(DEV).to(dt)
+    x = torch.randn(16, K, device=DEV, dtype=dt, requires_grad=True)
+    w = layer.weight
+    # what has to see the ops is not taken
+    with torch.device(DEV):                       # a function mode
+        assert not _module._plain_eager(x, w)
+    with torch.autograd.forward_ad.dual_level():
+        assert not _module._plain_eager(x, w)
+    torch.func.vmap(lambda t: (lambda _: t)(_flag(_module, t)))(x.detach())
+    assert not _module._plain_eager(x.cpu()) and not _module._plain_eager(torch.nn.Buffer(x.detach()).as_subclass(_Sub))
+    # saved-tensor hooks see what is kept; nothing is kept where no gradient is wanted
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or t.clone(), lambda t: t):
+        y = layer(x)
+    assert len(packed) >= 3
+    g1, = torch.autograd.grad(y.float().sum(), x, create_graph=True)
+    with pytest.raises(RuntimeError):             # no second derivative, and no silent zero either
+        g1.float().pow(2).sum().backward()
+    layer.requires_grad_(False)
+    assert not layer(x.detach()).requires_grad
+    g2, = torch.autograd.grad(layer(x).float().sum(), x)
+    assert torch.equal(g1, g2)
+    cp.check_device_status()
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def _flag(module, t):
+    assert not module._plain_eager(t)
+    return t
