@@ -251,8 +251,8 @@ extern "C" size_t prism_workspace_bytes(int kind, int M, int N, int K, int gs, i
   }
   if (gs <= 0 || rs <= 0 || N <= 0 || K <= 0) return bytes;
   const size_t G = (size_t)(N / gs);
-  // copy of R the kernels read: widened for rs = 8 (all kinds), halved for the gated dA+dR kernel
-  if (rs == 8) bytes += align256(G * 16 * (size_t)K * 2);
+  // copy of R the kernels read: widened for rs = 8 (the dB kernel does that itself), halved for the gated dA+dR kernel
+  if (rs == 8 && kind != PRISM_KIND_BWD_DB) bytes += align256(G * 16 * (size_t)K * 2);
   else if (kind == PRISM_KIND_BWD_DADR || kind == PRISM_KIND_BWD_DADR_IB) bytes += align256(G * (size_t)effective_block(rs) * K * 2);
   if (kind == PRISM_KIND_FWD) {
     // few tokens: the streaming forward keeps its arrival counters and fp32 partial sums here
@@ -410,13 +410,8 @@ extern "C" int prism_bwd_db_mask(const void* dC, const void* A, const void* R, c
   a.M = M; a.N = N; a.K = K; a.gs = gs; a.E = effective_block(rs);
   a.dtype = dtype; a.gate = gate; a.scale = dc_scale; a.out_f32 = db_f32;
   a.lddc = lddc; a.lda = lda; a.lddb = lddb;
-  a.R_eff = R; a.ldr = ldr;
+  a.R = R; a.ldr = ldr; a.widen = rs == 8 ? 1 : 0;
   uint8_t* wp = reinterpret_cast<uint8_t*>(workspace) + PRISM_WORKSPACE_HEADER_BYTES;
-  if (rs == 8) {
-    if ((rc = launch_expand_r8(R, wp, N / gs, K, ldr, dtype, s))) return rc;
-    a.R_eff = wp; a.ldr = K;
-    wp += align256((size_t)(N / gs) * 16 * K * 2);
-  }
   a.BN = (cfg && cfg[0] > 0) ? cfg[0] : default_bn(gs);
   if (a.BN % 16 != 0 || a.BN > 256 || gs % a.BN != 0)
     return fail(PRISM_ERR_BAD_ARG, "%s: tile BN=%d must be a multiple of 16, <= 256 and divide group_size=%d", fn, a.BN, gs);

@@ -10,7 +10,7 @@
 // and loads half of the dC columns) and a contiguous range of 128-token blocks.  The contraction of
 // the dense product runs over tokens, so both its operands are "MN-major": H tiles [128 tokens x 64
 // features] and dC tiles [128 tokens x 64 outputs] are used as the gate warps / TMA lay them out.
-//   warp 0      TMA: R_g tiles once; per token block two A tiles and ceil(BN/128) dC tiles
+//   warp 0      TMA: R_g tiles once (reconn_sz 8: all warps, from R itself, two 8 x 8 blocks widened to one of 16 x 16); per token block two A tiles and ceil(BN/128) dC tiles
 //   warps 1, 2  MMA issuers (leader), one per product.  Rotation S = A_blk . R_blk^T per rotation block
 //               as tcgen05.mma M256 N=2E K=16.  The two CTAs hold different features, hence different R blocks; an
 //               MMA spanning both takes its N rows half from each CTA, so it multiplies every row by
@@ -50,6 +50,8 @@ struct DbParams {
   int splits;
   int out_f32;        // 1: dB is fp32
   float scale;
+  const uint16_t* R8; // reconn_sz 8: R [G*8, K] itself, or null: the R tiles come through tmR
+  long long ldr;
   const void* ib;     // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
   uint32_t drop_thr;   // see drop_threshold
@@ -112,6 +114,17 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
   }
+  if (E == 16 && p.R8 != nullptr && threadIdx.x < 256) {
+    // Two tiles of 16 rows x 8 pieces (8 features): row i of the widened block holds R's row i % 8 in the pieces of parity
+    // i / 8.  A launch of its own for this copy cost 2 to 3 us before every call.
+    const int t = threadIdx.x >> 7, i = (threadIdx.x >> 3) & 15, c = threadIdx.x & 7;
+    const int col = f0 + t * 64 + c * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if ((c & 1) == (i >> 3) && col < p.K)
+      v = __ldg(reinterpret_cast<const uint4*>(p.R8 + (long long)(g * 8 + (i & 7)) * p.ldr + col));
+    *reinterpret_cast<uint4*>(smemR + t * p.r_tile_bytes + sw128_offset(i, c)) = v;
+    fence_proxy_async_smem();   // read by the rotation's MMAs, after the cluster barrier below
+  }
   if (warp == kWarpMma) {
     tmem_alloc_pair(&bars->tmem_base, 512);
     tmem_relinquish_pair();
@@ -133,12 +146,14 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       bool ok = true;
-      mbar_arrive_expect_tx(&bars->r_full, 2 * E * 128);
-      tma_load_2d(smemR, &tmR, &bars->r_full, f0, g * E);
-      tma_load_2d(smemR + p.r_tile_bytes, &tmR, &bars->r_full, f0 + 64, g * E);
-      // the rotation issuer (leader) reads the peer's R tiles too: it learns of them through the peer's
-      // first A tiles, which are issued after this wait
-      if (!mbar_wait(&bars->r_full, 0)) ok = false;
+      if (E != 16 || p.R8 == nullptr) {
+        mbar_arrive_expect_tx(&bars->r_full, 2 * E * 128);
+        tma_load_2d(smemR, &tmR, &bars->r_full, f0, g * E);
+        tma_load_2d(smemR + p.r_tile_bytes, &tmR, &bars->r_full, f0 + 64, g * E);
+        // the rotation issuer (leader) reads the peer's R tiles too: it learns of them through the peer's
+        // first A tiles, which are issued after this wait
+        if (!mbar_wait(&bars->r_full, 0)) ok = false;
+      }
       Ring rs(p.ns);
       for (int j = 0; j < nb && ok; ++j, rs.next()) {
         const int tok0 = (tb0 + j) * 128;
@@ -373,6 +388,7 @@ int launch_bwd_db(const DbArgs& a) {
   p.dc_tiles = (a.BN / 2 + 63) / 64;   // per CTA: half of the tile's dC columns
   p.r_tile_bytes = ((a.E * 128) + 1023) / 1024 * 1024;
   p.scale = a.scale; p.out_f32 = a.out_f32; p.ib = a.ib;
+  p.R8 = a.widen ? reinterpret_cast<const uint16_t*>(a.R) : nullptr; p.ldr = a.ldr;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
   p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_mask = a.drop_mask; p.n_k64 = (a.K + 63) / 64; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "bwd_db: dropout needs reconn_sz 8 or 16");
@@ -392,7 +408,7 @@ int launch_bwd_db(const DbArgs& a) {
   CUtensorMap tmA, tmR, tmdC;
   int rc;
   if ((rc = make_tmap_2d(&tmA, a.dtype, a.A, a.M, a.K, a.lda, 128, 64, true))) return rc;
-  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R_eff, (uint64_t)(a.N / a.gs) * a.E, a.K, a.ldr, a.E, 64, true))) return rc;
+  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R, (uint64_t)(a.N / a.gs) * (a.widen ? 8 : a.E), a.K, a.ldr, a.widen ? 8 : a.E, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmdC, a.dtype, a.dC, a.M, a.N, a.lddc, 128, 64, true))) return rc;
 
   using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, DbParams);

@@ -51,7 +51,8 @@ struct DbPlan {
 struct DbArgs {
   const void* dC;     // [M, N]
   const void* A;      // [M, K]
-  const void* R_eff;  // [(N/gs)*E, K]
+  const void* R;      // [(N/gs)*rs, K]
+  int widen;          // rs = 8: the kernel widens the blocks (E = 16)
   const void* ib;     // internal bias [N/gs, K] (gated modes) or null
   const long long* drop_seeds;  // [N/gs] per-group dropout seeds, or null
   float drop_p;
