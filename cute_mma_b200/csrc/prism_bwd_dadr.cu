@@ -5,90 +5,94 @@
 
 namespace prism {
 
-// dR[g*rs + i, k] = cast( scale * sum of the CTAs' partial sums ), in a fixed order: the main CTAs'
-// buffers in increasing order, then, for every run, the slabs of the extra pair that helped the
-// main pair (run, column of k).  For rs = 8 two neighbouring blocks share one 16-row group of the
-// partial buffers: the block in the upper 8 columns of each 16-column pair sits in rows 8..15.
+// The sums over CTAs that end the dA+dR call, in one launch: blocks [0, dr_blocks) form dR, the next d_ib_blocks the
+// internal-bias gradient, the rest dA (where the groups were split into parts).  A launch each cost 2 to 3 us of
+// device time, and more of host time where that is what a short step waits for.
+struct DadrReduce {
+  const float* partial;      // dR: see DadrParams
+  const float* partial_x;
+  void* dR;
+  long long lddr;
+  const float* partial_ib;   // d_ib: see DadrExtra
+  const float* partial_ib_x;
+  uint16_t* d_ib;
+  const float* partial_da;   // dA of the group parts [parts][M][K]
+  uint16_t* dA;
+  long long ldda;
+  int M, G, rs, E, K, runs, n_ft, n_main, n_extra, steal, slots, parts;
+  int k_blocks;              // blocks per row: 1024 columns each
+  unsigned dr_blocks, ib_blocks;
+  float scale, da_scale;
+};
+
+// Four neighbouring columns k.. of the sum over CTAs of `rows`-row buffers of K (main CTAs, in increasing order) and of 128
+// columns (for every run, the slabs of the extra pair that helped the main pair (run, column of k)).
+__device__ __forceinline__ float4 dadr_sum4(const DadrReduce& p, const float* main, const float* extra, long long rows,
+                                            long long row, int k) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [&](const float* src) {
+    const float4 v = *reinterpret_cast<const float4*>(src);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  };
+  for (int r = 0; r < 2 * p.runs; ++r) add(main + ((long long)r * rows + row) * p.K + k);
+  if (p.steal > 0) {
+    const int fx = k >> 7, kk = k & 127;
+    for (int run = 0; run < p.runs; ++run) {
+      const int m = run * p.n_ft + fx;
+      const int e = ((m + 1) * p.n_extra - 1) / p.n_main;   // the extra pair that helps main pair m
+      const int mi = m - e * p.n_main / p.n_extra;
+      for (int rank = 0; rank < 2; ++rank) add(extra + (((long long)(e * 2 + rank) * p.slots + mi) * rows + row) * 128 + kk);
+    }
+  }
+  return acc;
+}
+
+// dR[g*rs + i, k] = cast( scale * sum of the CTAs' partial sums ), in a fixed order.  For rs = 8 two neighbouring blocks
+// share one 16-row group of the partial buffers: the block in the upper 8 columns of each 16-column pair sits in rows
+// 8..15.  d_ib[g, k]: the CTAs' column sums of dS in the same order.  dA[m, k]: the parts' sums in part order.
+// One row, 1024 columns and four columns per thread (K is a multiple of 8).
 template <int DT, bool F32OUT>
-__global__ void dr_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ partial_x,
-                                 void* __restrict__ dR_out, int G, int rs, int E, int K, long long lddr, int runs,
-                                 int n_ft, int n_main, int n_extra, int steal, int slots, float scale) {
-  const long long pair = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)G * rs * K / 2;
-  if (pair >= total) return;
-  const long long idx = pair * 2;
-  const int k = (int)(idx % K);
-  const int row = (int)(idx / K);
-  const int g = row / rs, i = row - g * rs;
-  int ip = i;
-  if (rs == 8) ip = i + (((k & 15) >= 8) ? 8 : 0);
-  const long long GE = (long long)G * E;
-  const long long prow = (long long)g * E + ip;
-  float2 acc = make_float2(0.f, 0.f);
-  for (int r = 0; r < 2 * runs; ++r) {
-    const float2 v = *reinterpret_cast<const float2*>(partial + ((long long)r * GE + prow) * K + k);
-    acc.x += v.x;
-    acc.y += v.y;
-  }
-  if (steal > 0) {
-    const int fx = k >> 7, kk = k & 127;
-    for (int run = 0; run < runs; ++run) {
-      const int m = run * n_ft + fx;
-      const int e = ((m + 1) * n_extra - 1) / n_main;   // the extra pair that helps main pair m
-      const int mi = m - e * n_main / n_extra;
-      for (int rank = 0; rank < 2; ++rank) {
-        const float2 v = *reinterpret_cast<const float2*>(
-            partial_x + (((long long)(e * 2 + rank) * slots + mi) * GE + prow) * 128 + kk);
-        acc.x += v.x;
-        acc.y += v.y;
-      }
+__global__ void __launch_bounds__(256) dadr_reduce_kernel(const DadrReduce p) {
+  unsigned blk = blockIdx.x;
+  const bool is_dr = blk < p.dr_blocks;
+  if (!is_dr) blk -= p.dr_blocks;
+  const bool is_ib = !is_dr && blk < p.ib_blocks;
+  if (!is_dr && !is_ib) blk -= p.ib_blocks;
+  const int row = (int)(blk / p.k_blocks);
+  const int k = (int)(blk - (unsigned)row * p.k_blocks) * 1024 + threadIdx.x * 4;
+  if (k >= p.K) return;
+  float4 v;
+  float scale = p.scale;
+  uint16_t* dst;
+  if (is_dr) {
+    const int g = row / p.rs, i = row - g * p.rs;
+    const int ip = (p.rs == 8 && (k & 8)) ? i + 8 : i;
+    v = dadr_sum4(p, p.partial, p.partial_x, (long long)p.G * p.E, (long long)g * p.E + ip, k);
+    if (F32OUT) {   // the fp32 sums leave as they are (mixed-precision optimisers)
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dR) + (long long)row * p.lddr + k) =
+          make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+      return;
     }
-  }
-  if (F32OUT)   // the fp32 sums leave as they are (mixed-precision optimisers)
-    *reinterpret_cast<float2*>(reinterpret_cast<float*>(dR_out) + (long long)row * lddr + k) = make_float2(acc.x * scale, acc.y * scale);
-  else
-    *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dR_out) + (long long)row * lddr + k) = Elem<DT>::pack(acc.x * scale, acc.y * scale);
-}
-
-// d_ib[g, k] = cast( scale * sum of the CTAs' column sums of dS ), in the same fixed order as dR.
-template <int DT>
-__global__ void dib_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ partial_x,
-                                  uint16_t* __restrict__ d_ib, int G, int K, long long ldib, int runs, int n_ft,
-                                  int n_main, int n_extra, int steal, int slots, float scale) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)G * K) return;
-  const int k = (int)(idx % K), g = (int)(idx / K);
-  float acc = 0.f;
-  for (int r = 0; r < 2 * runs; ++r) acc += partial[((long long)r * G + g) * K + k];
-  if (steal > 0) {
-    const int fx = k >> 7, kk = k & 127;
-    for (int run = 0; run < runs; ++run) {
-      const int m = run * n_ft + fx;
-      const int e = ((m + 1) * n_extra - 1) / n_main;
-      const int mi = m - e * n_main / n_extra;
-      for (int rank = 0; rank < 2; ++rank)
-        acc += partial_x[(((long long)(e * 2 + rank) * slots + mi) * G + g) * 128 + kk];
+    dst = reinterpret_cast<uint16_t*>(p.dR) + (long long)row * p.lddr + k;
+  } else if (is_ib) {
+    v = dadr_sum4(p, p.partial_ib, p.partial_ib_x, p.G, row, k);
+    dst = p.d_ib + (long long)row * p.K + k;
+  } else {
+    const float4* src = reinterpret_cast<const float4*>(p.partial_da + (long long)row * p.K + k);
+    const long long step = (long long)p.M * p.K / 4;
+    v = __ldg(src);
+    for (int s = 1; s < p.parts; ++s) {
+      const float4 w = __ldg(src + s * step);
+      v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
     }
+    scale = p.da_scale;
+    dst = p.dA + (long long)row * p.ldda + k;
   }
-  d_ib[(long long)g * ldib + k] = (uint16_t)(Elem<DT>::pack(acc * scale, 0.f) & 0xffffu);
-}
-
-// dA[m, k] = cast( scale * sum over the group parts of partial[part][m][k] ), in part order; four elements per thread
-// (K is a multiple of 8).
-template <int DT>
-__global__ void __launch_bounds__(256) da_reduce_kernel(const float4* __restrict__ partial, uint16_t* __restrict__ dA, int M,
-                                                        int K, long long ldda, int parts, float scale) {
-  const int m = blockIdx.x;
-  const long long step = (long long)M * (K >> 2);
-  for (int c = threadIdx.x; c < (K >> 2); c += blockDim.x) {
-    const float4* src = partial + (long long)m * (K >> 2) + c;
-    float4 a = __ldg(src);
-    for (int s = 1; s < parts; ++s) {
-      const float4 v = __ldg(src + s * step);
-      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
-    }
-    *reinterpret_cast<uint2*>(dA + (long long)m * ldda + 4 * c) =
-        make_uint2(Elem<DT>::pack(a.x * scale, a.y * scale), Elem<DT>::pack(a.z * scale, a.w * scale));
+  const uint2 o = make_uint2(Elem<DT>::pack(v.x * scale, v.y * scale), Elem<DT>::pack(v.z * scale, v.w * scale));
+  if (is_ib && (reinterpret_cast<uintptr_t>(dst) & 7) != 0) {   // d_ib comes from the caller with no more than its own alignment
+    dst[0] = (uint16_t)o.x; dst[1] = (uint16_t)(o.x >> 16); dst[2] = (uint16_t)o.y; dst[3] = (uint16_t)(o.y >> 16);
+  } else {
+    *reinterpret_cast<uint2*>(dst) = o;
   }
 }
 
@@ -217,37 +221,26 @@ int launch_bwd_dadr(const DadrArgs& a) {
   dim3 grid(2 * (p.n_main + p.n_extra), a.grid.parts, 1);   // the two CTAs of a pair are neighbours
   kern<<<grid, dadr::kThreads, smem_bytes, a.stream>>>(tmA, tmRr, tmRd, tmdC, tmB, p, x);
   if ((rc = check_launch("prism_bwd_dadr"))) return rc;
-  if (a.grid.parts > 1) {
-    const int t = a.K >= 1024 ? 256 : ((a.K >> 2) + 31) / 32 * 32;
-    const float4* src = reinterpret_cast<const float4*>(a.partial_da);
-    uint16_t* dst = reinterpret_cast<uint16_t*>(a.dA);
-    if (a.dtype == DT_BF16) da_reduce_kernel<DT_BF16><<<a.M, t, 0, a.stream>>>(src, dst, a.M, a.K, a.ldda, a.grid.parts, a.scale);
-    else da_reduce_kernel<DT_F16><<<a.M, t, 0, a.stream>>>(src, dst, a.M, a.K, a.ldda, a.grid.parts, a.scale);
-    if ((rc = check_launch("prism_bwd_dadr dA reduce"))) return rc;
-  }
-
+  DadrReduce r;
+  r.partial = a.partial; r.partial_x = a.partial_x; r.dR = a.dR; r.lddr = a.lddr;
+  r.partial_ib = a.partial_ib; r.partial_ib_x = a.partial_ib_x; r.d_ib = reinterpret_cast<uint16_t*>(a.d_ib);
+  r.partial_da = a.partial_da; r.dA = reinterpret_cast<uint16_t*>(a.dA); r.ldda = a.ldda;
+  r.M = a.M; r.G = p.G; r.rs = a.rs; r.E = a.E; r.K = a.K; r.runs = p.runs; r.n_ft = p.n_ft; r.n_main = p.n_main;
+  r.n_extra = p.n_extra; r.steal = p.steal; r.slots = p.slots; r.parts = a.grid.parts;
   // gated mode: the kernel formed 2 dS against the halved R tiles, so the dR partials are doubled
-  const float r_scale = (a.gate != GATE_NONE) ? 0.5f * a.scale : a.scale;
-  const long long pairs = (long long)p.G * a.rs * a.K / 2;
-  const int threads = 256;
-  const long long blocks = (pairs + threads - 1) / threads;
-#define PRISM_DR_REDUCE(DT_, F32_)                                                                          \
-  dr_reduce_kernel<DT_, F32_><<<(unsigned)blocks, threads, 0, a.stream>>>(a.partial, a.partial_x, a.dR, p.G, a.rs, a.E, \
-      a.K, a.lddr, p.runs, p.n_ft, p.n_main, p.n_extra, p.steal, p.slots, r_scale)
-  if (a.dtype == DT_BF16) { if (a.dr_f32) PRISM_DR_REDUCE(DT_BF16, true); else PRISM_DR_REDUCE(DT_BF16, false); }
-  else { if (a.dr_f32) PRISM_DR_REDUCE(DT_F16, true); else PRISM_DR_REDUCE(DT_F16, false); }
-#undef PRISM_DR_REDUCE
-  if ((rc = check_launch("prism_bwd_dadr reduce"))) return rc;
-  if (ib) {
-    const long long n = (long long)p.G * a.K;
-    const long long nblocks = (n + threads - 1) / threads;
-    if (a.dtype == DT_BF16)
-      dib_reduce_kernel<DT_BF16><<<(unsigned)nblocks, threads, 0, a.stream>>>(a.partial_ib, a.partial_ib_x, reinterpret_cast<uint16_t*>(a.d_ib), p.G, a.K, a.K, p.runs, p.n_ft, p.n_main, p.n_extra, p.steal, p.slots, r_scale);
-    else
-      dib_reduce_kernel<DT_F16><<<(unsigned)nblocks, threads, 0, a.stream>>>(a.partial_ib, a.partial_ib_x, reinterpret_cast<uint16_t*>(a.d_ib), p.G, a.K, a.K, p.runs, p.n_ft, p.n_main, p.n_extra, p.steal, p.slots, r_scale);
-    return check_launch("prism_bwd_dadr internal-bias reduce");
-  }
-  return PRISM_OK;
+  r.scale = (a.gate != GATE_NONE) ? 0.5f * a.scale : a.scale;
+  r.da_scale = a.scale;
+  r.k_blocks = (a.K + 1023) / 1024;
+  const long long dr_blocks = (long long)p.G * a.rs * r.k_blocks, ib_blocks = ib ? (long long)p.G * r.k_blocks : 0;
+  const long long blocks = dr_blocks + ib_blocks + (a.grid.parts > 1 ? (long long)a.M * r.k_blocks : 0);
+  if (blocks > 0x7fffffffll) return fail(PRISM_ERR_UNSUPPORTED, "bwd_dadr: too many rows to reduce (%lld blocks)", blocks);
+  r.dr_blocks = (unsigned)dr_blocks; r.ib_blocks = (unsigned)ib_blocks;
+  const int threads = a.K >= 1024 ? 256 : ((a.K >> 2) + 31) / 32 * 32;
+#define PRISM_DADR_REDUCE(DT_, F32_) dadr_reduce_kernel<DT_, F32_><<<(unsigned)blocks, threads, 0, a.stream>>>(r)
+  if (a.dtype == DT_BF16) { if (a.dr_f32) PRISM_DADR_REDUCE(DT_BF16, true); else PRISM_DADR_REDUCE(DT_BF16, false); }
+  else { if (a.dr_f32) PRISM_DADR_REDUCE(DT_F16, true); else PRISM_DADR_REDUCE(DT_F16, false); }
+#undef PRISM_DADR_REDUCE
+  return check_launch("prism_bwd_dadr reduce");
 }
 
 }  // namespace prism

@@ -83,7 +83,7 @@ struct DadrParams {
 // fields inside DadrParams the instance without either (the benchmarked one) compiled to more spills.
 struct DadrExtra {
   // Few tiles (see dadr_groups_per_part): blockIdx.y splits the groups.  Part y walks groups [y g_per, (y + 1) g_per) and
-  // leaves fp32 sums for dA in partial_da [parts][M][K], which da_reduce_kernel adds; the parts' dR rows are disjoint.
+  // leaves fp32 sums for dA in partial_da [parts][M][K], which dadr_reduce_kernel adds; the parts' dR rows are disjoint.
   int g_per;           // groups per part (all of them: one part, dA written directly)
   float* partial_da;
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
