@@ -48,10 +48,6 @@ int launch_prep_r(const void* R, void* R_eff, int G, int rs, int E, int K, long 
   return check_launch("prep_r");
 }
 
-int launch_expand_r8(const void* R, void* R_eff, int G, int K, long long ldr, int dtype, cudaStream_t stream) {
-  return launch_prep_r(R, R_eff, G, 8, 16, K, ldr, 1.0f, dtype, stream);
-}
-
 // dbias[n] = sum over token rows of dC[m, n], in a fixed order: a block owns 256 columns and a
 // contiguous range of rows; its 8 warps take rows w, w + 8, ... (16-byte loads, 8 columns per lane)
 // and are added in warp order, then the row ranges are added in range order by the second kernel.
@@ -175,6 +171,15 @@ static int default_bn(int gs) {
   for (int c = 256; c >= 32; c -= 32)
     if (gs % c == 0) return c;
   return gs % 16 == 0 ? 16 : 0;
+}
+
+// Whether the general forward widens rotations of 8 itself or gets a widened copy of R from a launch before it (about 2 us,
+// and its host time): itself where a CTA pair has few chunks of 64 features to go through.  Measured, copy against
+// itself: 4 chunks 10.3 -> 9.1 us, 12 chunks 12.7 -> 11.9, 16 chunks 14.5 -> 13.9; 132 chunks (plain mode) 80 -> 78-81;
+// 448 chunks 269 -> 318, 448 of a deeper layer 228 -> 303.
+static bool fwd_widens(int M, int N, int K, int bn, int sms) {
+  const long long tiles = (long long)((M + 255) / 256) * (N / bn), pairs = sms / 2 > 0 ? sms / 2 : 1;
+  return (tiles + pairs - 1) / pairs * ((K + 63) / 64) <= 32;
 }
 
 static int check_common(const char* fn, int M, int N, int K, int gs, int rs, int dtype, int gate) {
@@ -351,13 +356,10 @@ extern "C" int prism_fwd_dropout(const void* A, const void* B, const void* R, co
   a.M = M; a.N = N; a.K = K; a.gs = gs; a.E = effective_block(rs);
   a.dtype = dtype; a.gate = gate;
   a.lda = lda; a.ldb = ldb; a.ldc = ldc;
-  a.R_eff = R; a.ldr = ldr;
+  a.R = R; a.ldr = ldr; a.widen = rs == 8 ? 1 : 0;
   uint8_t* wp = reinterpret_cast<uint8_t*>(workspace) + PRISM_WORKSPACE_HEADER_BYTES;
-  if (rs == 8) {
-    if ((rc = launch_expand_r8(R, wp, N / gs, K, ldr, dtype, s))) return rc;
-    a.R_eff = wp; a.ldr = K;
-    wp += align256((size_t)(N / gs) * 16 * K * 2);
-  }
+  uint8_t* r_copy = wp;
+  if (rs == 8) wp += align256((size_t)(N / gs) * 16 * K * 2);   // as prism_workspace_bytes lays it out
   a.num_sms = num_sms();
   a.err = reinterpret_cast<int*>(workspace);
   a.stream = s;
@@ -373,6 +375,10 @@ extern "C" int prism_fwd_dropout(const void* A, const void* B, const void* R, co
   a.sb = 0;
   if (a.BN % 16 != 0 || a.BN > 256 || gs % a.BN != 0)
     return fail(PRISM_ERR_BAD_ARG, "%s: tile BN=%d must be a multiple of 16, <= 256 and divide group_size=%d", fn, a.BN, gs);
+  if (a.widen && !fwd_widens(M, N, K, a.BN, a.num_sms)) {
+    if ((rc = launch_prep_r(R, r_copy, N / gs, rs, a.E, K, ldr, 1.0f, dtype, s))) return rc;
+    a.R = r_copy; a.ldr = K; a.widen = 0;
+  }
   return launch_fwd(a);
 }
 

@@ -10,7 +10,8 @@
 // owns 128 of the rows and loads half of the B tile, which halves the L2 traffic per flop.  Per CTA a
 // persistent loop over the pair's tiles.  One ring of shared-memory stages, one stage per 64-wide K
 // chunk: the A tile [128 x 64], this CTA's half of the R_g tile [E/2 x 64] and of the B_g tile [BN/2 x 64].
-//   warps 0, 2  TMA producers (A + R, B); 128-byte swizzle, zero fill outside the tensors
+//   warps 0, 2  TMA producers (A + R, B); 128-byte swizzle, zero fill outside the tensors.  reconn_sz 8: warp 0 writes the
+//               R tile itself, two 8 x 8 blocks of R widened to one of 16 x 16
 //   warp 1      MMA issuer (leader CTA only), per chunk
 //                 rotation  S = A_blk . R_blk^T per rotation block: tcgen05.mma M256 N=E K=16, fp32 into
 //                           one of four 64-column TMEM slots
@@ -60,6 +61,8 @@ struct FwdParams {
   int r_tile_bytes;     // bytes reserved for this CTA's half of the R tile (multiple of 1024)
   int stage_bytes;
   int tma_store;        // 1: epilogue goes through TMA stores (BN multiple of 64)
+  const uint16_t* R8;   // reconn_sz 8: R [G*8, K] itself, or null: the R tiles come through tmR
+  long long ldr;
   const void* bias;     // [N] or null
   const void* ib;       // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
@@ -151,7 +154,8 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxStages; ++i) {
-      mbar_init(&bars->loads_full[i], 4);   // two producers in each CTA, one arrive.expect_tx each
+      // two producers in each CTA, one arrive.expect_tx each (and one arrive for a R tile written by warp 0)
+      mbar_init(&bars->loads_full[i], (E == 16 && p.R8 != nullptr) ? 6 : 4);
       mbar_init(&bars->done[i], 1);
     }
     for (int i = 0; i < kSlots; ++i) {
@@ -161,6 +165,12 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     mbar_init(&bars->acc_full, 1);
     mbar_init(&bars->acc_empty, 2 * kNumEpiWarps);
     fence_mbar_init();
+  }
+  if (E == 16 && p.R8 != nullptr) {
+    // the blocks off the widened diagonal stay zero for good: the producer only writes the others
+    for (int i = threadIdx.x; i < p.ns * 64; i += kThreads)
+      *reinterpret_cast<uint4*>(smemSt + (i >> 6) * p.stage_bytes + kATileBytes + (i & 63) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async_smem();
   }
   if (warp == kWarpMma) {
     tmem_alloc_pair(&bars->tmem_base, 512);
@@ -183,7 +193,44 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int my_tiles = (p.n_tiles - cid + n_clusters - 1) / n_clusters;
   const uint32_t total = (uint32_t)my_tiles * nk;   // chunks this CTA pair processes
 
-  if (warp == kWarpTma) {
+  if (E == 16 && warp == kWarpTma && p.R8 != nullptr) {
+    // ------------------------------------------------------------------ producer for reconn_sz 8: A tile by TMA, R by hand
+    // This CTA's eight rows of the widened R tile are R's eight rows of the group in every second piece of 8 features
+    // (the leader the even ones, the peer the odd ones): one 16-byte piece per lane, fetched a chunk ahead.  For
+    // short calls only (see fwd_widens): a chunk takes this warp longer than the TMA path.
+    Ring rs(p.ns);
+    int t = cid, c = 0, mt, nt;
+    tile_coords(p, t, mt, nt);
+    const int r_row = lane >> 2, r_piece = (lane & 3) * 2 + (int)rank;
+    const uint32_t r_dst = kATileBytes + sw128_offset(r_row, r_piece);
+    auto fetch = [&](int nt_, int c_) {
+      const int col = c_ * 64 + r_piece * 8;
+      const long long row = (long long)(nt_ / p.ntiles_per_group) * 8 + r_row;
+      return col < p.K ? __ldg(reinterpret_cast<const uint4*>(p.R8 + row * p.ldr + col)) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    uint4 r_next = total > 0 ? fetch(nt, 0) : make_uint4(0u, 0u, 0u, 0u);
+    bool ok = true;
+    for (uint32_t j = 0; j < total; ++j, rs.next()) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->done[rs.idx], rs.phase ^ 1))) { ok = false; break; }
+      uint8_t* dst = smemSt + rs.idx * p.stage_bytes;
+      const uint32_t full = mapa_shared(smem_u32(&bars->loads_full[rs.idx]), 0);
+      if (lane == 0) {
+        mbar_arrive_expect_tx_cluster(full, kATileBytes);
+        tma_load_2d_pair(dst, &tmA, full, c * 64, mt * 256 + (int)rank * 128);
+      }
+      *reinterpret_cast<uint4*>(dst + r_dst) = r_next;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(full);
+      if (++c == nk) {
+        c = 0;
+        t += n_clusters;
+        if (t < p.n_tiles) tile_coords(p, t, mt, nt);
+      }
+      if (j + 1 < total) r_next = fetch(nt, c);
+    }
+    if (!ok && lane == 0) { atomicExch(p.err, PRISM_ERR_DEVICE_WAIT); }
+  } else if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA producer: A tile and half of the R tile
     if (lane == 0) {
       Ring rs(p.ns);
@@ -457,6 +504,7 @@ int launch_fwd(const FwdArgs& a) {
   p.n_kchunks = (a.K + 63) / 64;
   p.r_tile_bytes = ((a.E / 2 * 128) + 1023) / 1024 * 1024;   // this CTA's E/2 rows of the R tile
   p.tma_store = (a.BN % 64 == 0) ? 1 : 0;
+  p.R8 = a.widen ? reinterpret_cast<const uint16_t*>(a.R) : nullptr; p.ldr = a.ldr;
   p.bias = a.bias; p.ib = a.ib; p.C = a.C; p.ldc = a.ldc; p.err = a.err;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
   p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
@@ -476,7 +524,7 @@ int launch_fwd(const FwdArgs& a) {
   CUtensorMap tmA, tmR, tmB, tmC;
   int rc;
   if ((rc = make_tmap_2d(&tmA, a.dtype, a.A, a.M, a.K, a.lda, 128, 64, true))) return rc;
-  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R_eff, (uint64_t)(a.N / a.gs) * a.E, a.K, a.ldr, a.E / 2, 64, true))) return rc;
+  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R, (uint64_t)(a.N / a.gs) * (a.widen ? 8 : a.E), a.K, a.ldr, a.E / 2, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmB, a.dtype, a.B, a.N, a.K, a.ldb, a.BN / 2, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmC, a.dtype, a.C, a.M, a.N, a.ldc, 32, 64, true))) return rc;
 

@@ -48,6 +48,8 @@ struct FwdSmallParams {
   int units, ncta;     // G * nk work units over ncta CTAs
   int pmax;            // partial slots per group
   int ns, stage_bytes, a_off, r_off, b_off;
+  const uint16_t* R8;  // reconn_sz 8: R [G*8, K] itself, or null: the R tiles come through tmR
+  long long ldr;
   const void* bias;
   const void* ib;      // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
@@ -118,6 +120,12 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmR);
   }
+  if (E == 16 && p.R8 != nullptr) {
+    // the blocks off the widened diagonal stay zero for good: the rotation's warp only writes the others
+    for (int i = threadIdx.x; i < p.ns * 128; i += kThreads)
+      *reinterpret_cast<uint4*>(smemSt + (i >> 7) * p.stage_bytes + p.r_off + (i & 127) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async_smem();
+  }
   if (warp == kWarpMma) {
     tmem_alloc_cta(&bars->tmem_base, 512);
     tmem_relinquish_cta();
@@ -125,7 +133,8 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   // the producer fills the ring's first pass before the CTA-wide synchronisation: nothing else has
   // touched these stages yet, so their "empty" barriers need no wait
   const uint64_t pol = l2_policy_evict_first();
-  const uint32_t stage_tx = (uint32_t)(p.nrt * kTile + p.Mp * 128 + E * 128);
+  const bool widen = E == 16 && p.R8 != nullptr;   // reconn_sz 8: the rotation's warp writes the R tile
+  const uint32_t stage_tx = (uint32_t)(p.nrt * kTile + p.Mp * 128 + (widen ? 0 : E * 128));
   int pre = 0;
   if (threadIdx.x == 0) {
     int g = u0 / p.nk, kc = u0 - g * p.nk;
@@ -135,7 +144,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       for (int j = 0; j < p.nrt; ++j)
         tma_load_2d_hint(dst + p.b_off + j * kTile, &tmB, &bars->full[pre], kc * 64, g * p.gs + j * 128, pol);
       tma_load_2d(dst + p.a_off, &tmA, &bars->full[pre], kc * 64, 0);
-      tma_load_2d(dst + p.r_off, &tmR, &bars->full[pre], kc * 64, g * E);
+      if (!widen) tma_load_2d(dst + p.r_off, &tmR, &bars->full[pre], kc * 64, g * E);
       if (++kc == p.nk) { kc = 0; ++g; }
     }
   }
@@ -161,14 +170,28 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         for (int j = 0; j < p.nrt; ++j)
           tma_load_2d_hint(dst + p.b_off + j * kTile, &tmB, &bars->full[rs.idx], kc * 64, g * p.gs + j * 128, pol);
         tma_load_2d(dst + p.a_off, &tmA, &bars->full[rs.idx], kc * 64, 0);
-        tma_load_2d(dst + p.r_off, &tmR, &bars->full[rs.idx], kc * 64, g * E);
+        if (!widen) tma_load_2d(dst + p.r_off, &tmR, &bars->full[rs.idx], kc * 64, g * E);
         if (++kc == p.nk) { kc = 0; ++g; }
       }
       if (!ok) atomicExch(p.err, PRISM_ERR_DEVICE_WAIT);
     }
   } else if (warp == kWarpRot) {
     // ------------------------------------------------------------------ MMA issuer 1: rotation S = A_chunk . R_g^T
-    if (lane == 0) {
+    // reconn_sz 8: the warp first writes the unit's R tile, two 8 x 8 blocks of R widened to one of 16 x 16.  Row i of the
+    // widened blocks is R's row i % 8 in the pieces of 8 features of parity i / 8: two 16-byte pieces per lane, fetched a
+    // unit ahead.  (A launch of its own for the widened copy: 2.2 us of 19 for 20 tokens, 1024 -> 16384.)
+    if (lane == 0 || widen) {
+      const int r_row = lane >> 2, r_piece = (lane & 3) * 2;   // and row + 8, piece + 1
+      int gr = u0 / p.nk, kr = u0 - gr * p.nk;
+      uint4 r_even = make_uint4(0u, 0u, 0u, 0u), r_odd = r_even;
+      auto fetch = [&]() {
+        const uint16_t* src = p.R8 + ((long long)gr * 8 + r_row) * p.ldr + kr * 64 + r_piece * 8;
+        const int col = kr * 64 + r_piece * 8;
+        r_even = col < p.K ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(0u, 0u, 0u, 0u);
+        r_odd = col + 8 < p.K ? __ldg(reinterpret_cast<const uint4*>(src) + 1) : make_uint4(0u, 0u, 0u, 0u);
+        if (++kr == p.nk) { kr = 0; ++gr; }
+      };
+      if (widen && u0 < u1) fetch();
       const uint32_t idesc_r = make_idesc(DT, 128, E, 0, 0);        // S block: M = 128 token rows, N = E
       const uint64_t d0 = desc_kmajor_sw128(smem_u32(smemSt), 1024);
       const uint32_t d_hi = (uint32_t)(d0 >> 32);
@@ -180,9 +203,20 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       for (int i = 0; i < n; ++i, rl.next()) {
         const uint32_t slot = (uint32_t)i & 1u;
         if (i >= 2) {   // the gate warps hold S of unit i - 2 in registers
-          if (!mbar_wait(&bars->s_free[slot], (((uint32_t)i >> 1) - 1) & 1)) { ok = false; break; }
+          const bool got = mbar_wait(&bars->s_free[slot], (((uint32_t)i >> 1) - 1) & 1);
+          if (widen ? !__all_sync(0xffffffffu, got) : !got) { ok = false; break; }
         }
-        if (!mbar_wait(&bars->full[rl.idx], rl.phase)) { ok = false; break; }
+        const bool got = mbar_wait(&bars->full[rl.idx], rl.phase);
+        if (widen ? !__all_sync(0xffffffffu, got) : !got) { ok = false; break; }
+        if (widen) {   // the stage is this unit's, the rotation that read its R tile before has long completed
+          uint8_t* rt = smemSt + rl.idx * p.stage_bytes + p.r_off;
+          *reinterpret_cast<uint4*>(rt + sw128_offset(r_row, r_piece)) = r_even;
+          *reinterpret_cast<uint4*>(rt + sw128_offset(r_row + 8, r_piece + 1)) = r_odd;
+          if (i + 1 < n) fetch();
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane != 0) continue;
+        }
         tc_fence_after_sync();
         const uint32_t base = (uint32_t)d0 + rl.idx * st_step;
 #pragma unroll
@@ -379,6 +413,7 @@ int launch_fwd_small(const FwdArgs& a, void* scratch) {
   p.nrt = a.gs / 128;
   p.nk = (a.K + 63) / 64;
   fwd_small_partition(p.G, p.nk, a.num_sms, &p.units, &p.ncta, &p.pmax);
+  p.R8 = a.widen ? reinterpret_cast<const uint16_t*>(a.R) : nullptr; p.ldr = a.ldr;
   p.bias = a.bias; p.ib = a.ib; p.C = a.C; p.ldc = a.ldc; p.err = a.err;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
   p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
@@ -399,7 +434,7 @@ int launch_fwd_small(const FwdArgs& a, void* scratch) {
   CUtensorMap tmA, tmR, tmB;
   int rc;
   if ((rc = make_tmap_2d(&tmA, a.dtype, a.A, a.M, a.K, a.lda, p.Mp, 64, true))) return rc;
-  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R_eff, (uint64_t)p.G * a.E, a.K, a.ldr, a.E, 64, true))) return rc;
+  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R, (uint64_t)p.G * (a.widen ? 8 : a.E), a.K, a.ldr, a.widen ? 8 : a.E, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmB, a.dtype, a.B, a.N, a.K, a.ldb, 128, 64, true))) return rc;
 
   using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FwdSmallParams);

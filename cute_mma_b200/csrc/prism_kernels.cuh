@@ -11,7 +11,8 @@ namespace prism {
 struct FwdArgs {
   const void* A;      // [M, K]
   const void* B;      // [N, K]
-  const void* R_eff;  // [(N/gs)*E, K]  rotation blocks padded to E x E
+  const void* R;      // [(N/gs)*rs, K]
+  int widen;          // rs = 8: the kernel widens two blocks to one of 16 x 16 (E = 16); 0: R holds E-wide blocks
   const void* bias;   // [N] or null
   const void* ib;     // internal bias [N/gs, K] (gated modes) or null
   const long long* drop_seeds;  // [N/gs] per-group dropout seeds, or null (no dropout)
@@ -35,10 +36,8 @@ bool fwd_small_preferred(int M);   // token counts for which it is the default c
 size_t fwd_small_scratch_bytes(int M, int N, int K, int gs, int num_sms);
 int launch_fwd_small(const FwdArgs& a, void* scratch);
 
-// R [(G*8), K] -> R_eff [(G*16), K]: two neighbouring 8x8 blocks become one 16x16
-// block-diagonal block, so that every rotation is a 16-wide tensor-core product.
-int launch_expand_r8(const void* R, void* R_eff, int G, int K, long long ldr, int dtype, cudaStream_t stream);
-// R_eff [(G*E), K] = factor * R (widened as above when rs = 8)
+// Copy of R for the dA+dR kernel and long forwards: R_eff [(G*E), K] = factor * R; rs = 8: two neighbouring 8x8 blocks become one
+// block-diagonal 16x16 block, so that every rotation is a 16-wide tensor-core product.
 int launch_prep_r(const void* R, void* R_eff, int G, int rs, int E, int K, long long ldr, float factor, int dtype,
                   cudaStream_t stream);
 

@@ -250,3 +250,19 @@ def test_reductions_of_dadr_share_a_launch(K, rs):
         cp.check_device_status()
         assert torch.equal(dA, dA2) and torch.equal(dib, dib2) and torch.equal(dR.to(dt), dR2)
         assert O.rel_err(dA.float(), ref[0]) < TOL and O.rel_err(dR, ref[1]) < TOL and O.rel_err(dib.float(), ref[3]) < TOL
+
+
+@pytest.mark.parametrize("M,path", [(1, 2), (100, 2), (100, 1), (700, 1)])    # the streaming kernel and the general one
+@pytest.mark.parametrize("K", [8, 72, 136, 1000])                             # one block; odd counts of blocks; a ragged chunk
+@pytest.mark.parametrize("act", [None, "silu_gate"])
+def test_rotations_of_8_are_widened_in_the_forward(M, K, path, act):
+    """More chunks than stages and more tiles than CTA pairs; non-finite values in one block reach that block only."""
+    gs, rs, dt = 128, 8, torch.bfloat16
+    N = gs * (200 if K < 100 else 600 if M == 700 else 9)   # the last: long enough for the copy
+    A, B, R, _ = _inputs(M, K, N, gs, rs, dt, 19)
+    C, _ = cp.forward(A, B, R, gs, rs, activation=act, tile_cfg=[0, 0, 0, path])
+    cp.check_device_status()
+    assert O.rel_err(C.float(), O.prism_forward(A.float(), B.float(), R.float(), gs, rs, act)) < TOL
+    R[:8, :8] = float("inf")                     # the first block of group 0
+    C2, _ = cp.forward(A, B, R, gs, rs, activation=act, tile_cfg=[0, 0, 0, path])
+    assert torch.equal(C2[:, gs:], C[:, gs:])
