@@ -173,6 +173,16 @@ static int default_bn(int gs) {
   return gs % 16 == 0 ? 16 : 0;
 }
 
+// n-tile of the general forward: the widest, halved (down to 64) as long as the narrower tiles still run in one wave.  A
+// narrow tile repeats its group's rotation and gate, but on a CTA pair that would be idle, and its epilogue is shorter.
+// Measured, 256 against 64 wide: 1024 x 256 -> 1024 8.9 / 7.1 us, 1024 x 768 -> 768 12.8 / 10.7; 200 x 4096 -> 1024 32.6 /
+// 30.4; 32 wide is no faster (8.8, 15.7, 30.3), and two waves lose (128 x 4096 -> 14336: 36.7 / 104.9).
+static int fwd_default_bn(int M, int N, int gs, int sms) {
+  int bn = default_bn(gs);
+  while (bn % 64 == 0 && bn >= 128 && (long long)((M + 255) / 256) * (N / (bn / 2)) <= sms / 2) bn /= 2;
+  return bn;
+}
+
 // Whether the general forward widens rotations of 8 itself or gets a widened copy of R from a launch before it (about 2 us,
 // and its host time): itself where a CTA pair has few chunks of 64 features to go through.  Measured, copy against
 // itself: 4 chunks 10.3 -> 9.1 us, 12 chunks 12.7 -> 11.9, 16 chunks 14.5 -> 13.9; 132 chunks (plain mode) 80 -> 78-81;
@@ -369,7 +379,7 @@ extern "C" int prism_fwd_dropout(const void* A, const void* B, const void* R, co
     return fail(PRISM_ERR_UNSUPPORTED, "%s: the few-token kernel needs M <= 128 and group_size a multiple of 128 (M=%d, group_size=%d)", fn, M, gs);
   if (path != 1 && fwd_small_supported(M, N, K, gs, a.E) && (path == 2 || fwd_small_preferred(M)))
     return launch_fwd_small(a, wp);
-  a.BN = (cfg && cfg[0] > 0) ? cfg[0] : default_bn(gs);
+  a.BN = (cfg && cfg[0] > 0) ? cfg[0] : fwd_default_bn(M, N, gs, a.num_sms);
   a.PM = (cfg && cfg[1] > 0) ? cfg[1] : 16;
   a.sa = (cfg && cfg[2] > 0) ? cfg[2] : 0;
   a.sb = 0;

@@ -266,3 +266,16 @@ def test_rotations_of_8_are_widened_in_the_forward(M, K, path, act):
     R[:8, :8] = float("inf")                     # the first block of group 0
     C2, _ = cp.forward(A, B, R, gs, rs, activation=act, tile_cfg=[0, 0, 0, path])
     assert torch.equal(C2[:, gs:], C[:, gs:])
+
+
+@pytest.mark.parametrize("M,N,gs", [(1, 256, 256), (257, 1024, 256), (256, 18944, 256), (300, 768, 192), (64, 512, 512)])
+def test_tile_width_of_short_forwards(M, N, gs):
+    """Narrow tiles while they fit one wave (74 tiles of 256: none; groups of 192: 96 wide) give the bits of wide ones."""
+    K, rs, dt = 200, 8, torch.float16
+    A, B, R, _ = _inputs(M, K, N, gs, rs, dt, 21)
+    bias = torch.randn(N, device=DEV).to(dt)
+    C, _ = cp.forward(A, B, R, gs, rs, activation="silu_gate", bias=bias, tile_cfg=[0, 0, 0, 1])
+    wide, _ = cp.forward(A, B, R, gs, rs, activation="silu_gate", bias=bias, tile_cfg=[192 if gs == 192 else 256, 0, 0, 1])
+    cp.check_device_status()
+    assert torch.equal(C, wide)
+    assert O.rel_err(C.float(), O.prism_forward(A.float(), B.float(), R.float(), gs, rs, "silu_gate", bias=bias.float())) < TOL
