@@ -104,9 +104,17 @@ class ShuffleFold:
         self.inv = inv.to(device)
         self.inv_in_chunk = (inv.view(G, n_chunks, 64) % 64).to(device)       # the same, inside its chunk
         self.perm_in_chunk = (perm.view(G, n_chunks, 64) % 64).to(device)
-        # the same per segment of two features, as the copy kernels take it
+        self._segments()
+
+    def _segments(self):
+        """The maps per segment of two features, as the copy kernels take them."""
         self.inv_seg = (self.inv_in_chunk[:, :, ::2] // 2).to(torch.uint8).contiguous()
         self.perm_seg = (self.perm_in_chunk[:, :, ::2] // 2).to(torch.uint8).contiguous()
+
+    def __setstate__(self, state):   # a layer pickled before the segment tables existed brings the other maps only
+        self.__dict__.update(state)
+        if "inv_seg" not in state:
+            self._segments()
 
     def _native(self, X: torch.Tensor, rows: int, sizes=(2,)) -> bool:
         """Whether the library's copy kernels take X: on this fold's GPU, elements of 2 (or 4) bytes, whole rows;

@@ -215,3 +215,15 @@ def test_input_shuffle_fold_is_the_reference_shuffle():
         Rq = R.clone().requires_grad_(True)
         (fold.fold_R(Rq) * gf[1]).sum().backward()
         assert (Rq.grad - fold.unfold_dR(gf[1])).abs().max() < 1e-12
+
+
+def test_shuffle_fold_pickles_of_both_forms():
+    import copy
+    import pickle
+    from cute_mma_b200 import _shuffle as S
+    masks, _ = S.build_shuffle_masks(128, 96, 32, 16)
+    fold = S.ShuffleFold(masks, 128, 32, 16, "cpu")
+    old = copy.copy(fold)
+    del old.inv_seg, old.perm_seg               # as a layer pickled before the segment tables existed brings it
+    for f in (pickle.loads(pickle.dumps(fold)), pickle.loads(pickle.dumps(old))):
+        assert torch.equal(f.inv_seg, fold.inv_seg) and torch.equal(f.perm_seg, fold.perm_seg)
