@@ -19,7 +19,8 @@
 //   warps 4-19  gate warps, 16 token rows x 64 features each: S from TMEM, A by ldmatrix, H = A*silu(S)
 //               on registers, stmatrix of H over the A tile in place
 //               Dense product D += H^T . dC as 8 x tcgen05.mma M256 N=BN K=16 per token block.
-//   warps 20-23 epilogue: D -> dB (transposed store), or fp32 partials when the token range is split;
+//   warps 20-23 epilogue: D -> dB (transposed by stmatrix into the stages' memory, TMA stores), fp32 dB, or fp32
+//               partials when the token range is split;
 //               a second kernel then adds the partials in a fixed order (deterministic).
 // Both products run on tcgen05: mma.sync would share the tensor cores with tcgen05.mma and starve
 // behind it.
@@ -49,6 +50,7 @@ struct DbParams {
   int stage_bytes;
   int splits;
   int out_f32;        // 1: dB is fp32
+  int box_rows;       // rows of dB per TMA store of the epilogue (divides BN)
   float scale;
   const uint16_t* R8; // reconn_sz 8: R [G*8, K] itself, or null: the R tiles come through tmR
   long long ldr;
@@ -80,7 +82,7 @@ struct DbBarriers {
 template <int DT, int GATE, int E, bool DROP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(db::kThreads, 1)
 prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmR,
-                    const __grid_constant__ CUtensorMap tmdC, const DbParams p) {
+                    const __grid_constant__ CUtensorMap tmdC, const __grid_constant__ CUtensorMap tmdB, const DbParams p) {
   using namespace db;
   constexpr int KS = E / 16;    // K16 steps per rotation block
   constexpr int NBLK = 128 / E; // rotation blocks of this CTA's 128 features
@@ -276,7 +278,45 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int q = warp & 3;
     const int f = f0 + q * 32 + lane;  // feature = accumulator row
     bool ok = mbar_wait(&bars->acc_full, 0);
-    if (ok) {
+    if (p.splits == 1 && !p.out_f32) {
+      // Every product has completed, so the stages' memory is free: box_rows rows of dB (outputs) by 2 x 64 features at a
+      // time go there, each warp's 32 features transposed by stmatrix, and leave by TMA.  Two-byte stores from
+      // the accumulator's rows, 64 bytes per instruction, took 1.3 us more per tile: 128 x 4096 -> 14336 118 -> 102 us,
+      // 2048 x 4096 -> 14336 316 -> 300, 8192 x 1024 -> 16384 292 -> 290.
+      const uint32_t mat = lane >> 3, l8 = lane & 7;
+      const uint32_t stage = smem_u32(smemSt);
+      const uint32_t box_bytes = (uint32_t)p.box_rows * 128;
+      const uint32_t piece0 = (q & 1) * 4 + (mat & 1);   // this lane's 16-byte piece of a row, for the lower 16 features
+      const uint32_t row0 = (mat >> 1) * 8 + l8;         // ... and its row, inside 16
+      const uint32_t tacc = tmem_base + (uint32_t(q * 32) << 16);
+      if (ok) tc_fence_after_sync();
+      for (int c0 = 0, blk = 0; c0 < p.BN; c0 += p.box_rows, ++blk) {
+        const uint32_t tile = stage + (2 * blk + (q >> 1)) * box_bytes;
+        for (int r = 0; ok && r < p.box_rows; r += 16) {
+          uint32_t v[2][8];
+          tmem_ld_16x256b_x2(tacc + c0 + r, v[0]);
+          tmem_ld_16x256b_x2(tacc + (16u << 16) + c0 + r, v[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[e] = Elem<DT>::pack(__uint_as_float(v[h][2 * e]) * p.scale, __uint_as_float(v[h][2 * e + 1]) * p.scale);
+            stmatrix_x4_trans(tile + sw128_offset(r + row0, piece0 + 2 * h), w);
+          }
+        }
+        fence_proxy_async_smem();
+        // the four epilogue warps, whether their wait ran out or not
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (ok && lane == 0 && q < 2 && f0 + q * 64 < p.K) {
+          tma_store_2d(&tmdB, smemSt + (2 * blk + q) * box_bytes, f0 + q * 64, n0 + c0);
+          tma_store_commit();
+        }
+      }
+      if (lane == 0 && q < 2) tma_store_wait_all<0>();   // outstanding stores read shared memory
+      if (!ok && lane == 0) atomicExch(p.err, PRISM_ERR_DEVICE_WAIT);
+    } else if (ok) {
       tc_fence_after_sync();
       for (int c0 = 0; c0 < p.BN; c0 += 16) {
         uint32_t v[16];
@@ -287,17 +327,10 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             float* dst = p.partial + ((long long)split * p.part_rows + (n0 - p.nt0 * p.BN) + c0) * p.K + f;
 #pragma unroll
             for (int j = 0; j < 16; ++j) dst[(long long)j * p.K] = __uint_as_float(v[j]) * p.scale;
-          } else if (p.out_f32) {
+          } else {
             float* dst = reinterpret_cast<float*>(p.dB) + (long long)(n0 + c0) * p.lddb + f;
 #pragma unroll
             for (int j = 0; j < 16; ++j) dst[(long long)j * p.lddb] = __uint_as_float(v[j]) * p.scale;
-          } else {
-            uint16_t* dst = reinterpret_cast<uint16_t*>(p.dB) + (long long)(n0 + c0) * p.lddb + f;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const uint32_t w = Elem<DT>::pack(__uint_as_float(v[j]) * p.scale, 0.f);
-              dst[(long long)j * p.lddb] = static_cast<uint16_t>(w & 0xFFFFu);
-            }
           }
         }
       }
@@ -405,13 +438,17 @@ int launch_bwd_db(const DbArgs& a) {
   p.ns = ns;
   const int smem_bytes = 2 * p.r_tile_bytes + ns * p.stage_bytes + (int)sizeof(DbBarriers) + 1024;
 
-  CUtensorMap tmA, tmR, tmdC;
+  CUtensorMap tmA, tmR, tmdC, tmdB;
   int rc;
   if ((rc = make_tmap_2d(&tmA, a.dtype, a.A, a.M, a.K, a.lda, 128, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmR, a.dtype, a.R, (uint64_t)(a.N / a.gs) * (a.widen ? 8 : a.E), a.K, a.ldr, a.widen ? 8 : a.E, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmdC, a.dtype, a.dC, a.M, a.N, a.lddc, 128, 64, true))) return rc;
 
-  using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, DbParams);
+  p.box_rows = a.BN % 64 == 0 ? 64 : a.BN % 32 == 0 ? 32 : 16;
+  if (a.out_f32) tmdB = tmdC;   // not used
+  else if ((rc = make_tmap_2d(&tmdB, a.dtype, a.dB, a.N, a.K, a.lddb, p.box_rows, 64, true))) return rc;
+
+  using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, DbParams);
   KernT kern = nullptr;
 #define PRISM_PICK_G(DT_, E_, DROP_)                                                                    \
   (a.gate == GATE_SILU ? (KernT)prism_bwd_db_kernel<DT_, GATE_SILU, E_, DROP_>                           \
@@ -431,7 +468,7 @@ int launch_bwd_db(const DbArgs& a) {
     q.blocks_per_split = (p.n_tokblocks + splits - 1) / splits;
     q.splits = (p.n_tokblocks + q.blocks_per_split - 1) / q.blocks_per_split;   // drop splits that would own no token block
     dim3 grid(2 * ((a.K + 255) / 256), nrows, q.splits);   // x: CTA pairs of 2 x 128 features
-    kern<<<grid, db::kThreads, smem_bytes, a.stream>>>(tmA, tmR, tmdC, q);
+    kern<<<grid, db::kThreads, smem_bytes, a.stream>>>(tmA, tmR, tmdC, tmdB, q);
     int rcl;
     if ((rcl = check_launch("prism_bwd_db"))) return rcl;
     if (q.splits > 1) {

@@ -279,3 +279,19 @@ def test_tile_width_of_short_forwards(M, N, gs):
     cp.check_device_status()
     assert torch.equal(C, wide)
     assert O.rel_err(C.float(), O.prism_forward(A.float(), B.float(), R.float(), gs, rs, "silu_gate", bias=bias.float())) < TOL
+
+
+@pytest.mark.parametrize("gs,N", [(16, 48), (32, 64), (96, 192), (256, 512)])   # stores of 16, 32 and 64 rows of dB
+@pytest.mark.parametrize("K", [8, 72, 200, 328])                                 # features that end inside a 64-wide store
+def test_transposed_stores_of_db(gs, N, K):
+    """16-bit dB is the rounded fp32 dB, which leaves by plain stores, and touches nothing beside it."""
+    from cute_mma_b200 import _functional as F
+    M, rs, dt = 128, 8, torch.bfloat16
+    A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 23)
+    pad = torch.full((N + 2, K), 7.0, dtype=dt, device=DEV)
+    dB = F._backward_db(dC, A, R, gs, rs, 1, dc_scale=0.5, dB_out=pad[1:N + 1])
+    wide = F._backward_db(dC, A, R, gs, rs, 1, dc_scale=0.5, out_dtype=torch.float32)
+    cp.check_device_status()
+    assert torch.equal(dB, wide.to(dt)) and (pad[0] == 7).all() and (pad[N + 1] == 7).all()
+    ref = O.prism_backward(0.5 * dC.float(), A.float(), B.float(), R.float(), gs, rs, "silu_gate")[2]
+    assert O.rel_err(wide, ref) < TOL
