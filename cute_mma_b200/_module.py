@@ -256,7 +256,8 @@ class _LayerFn(torch.autograd.Function):
         A, weight, R, ib, P = ctx.saved_tensors
         group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, has_bias, seeds = ctx.args
         rs = reconn_sz if fold is None else 64
-        dC = dC.contiguous()
+        # the kernels take whole rows; saved-tensor hooks may hand back views of another layout
+        dC, A, weight, R = dC.contiguous(), A.contiguous(), weight.contiguous(), R.contiguous()
         gate = F._gate_code(activation or None)
         ib = None if ib is None else ib.contiguous()
         need_dB = ctx.needs_input_grad[1]

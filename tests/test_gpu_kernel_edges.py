@@ -227,6 +227,23 @@ def test_eager_layer_under_autograd_features():
     cp.check_device_status()
 
 
+@pytest.mark.parametrize("kw", [dict(activation="silu_gate", internal_bias=True), dict()])   # the second: Cayley
+def test_unpacked_views_of_another_layout(kw):
+    """Saved-tensor hooks that hand back every second element of a wider buffer: the gradients of the plain call."""
+    K, N, dt = 128, 256, torch.bfloat16
+    layer = cp.PrismLinear(K, N, group_size=64, reconn_sz=8, **kw).to(DEV).to(dt)
+    torch.nn.init.normal_(layer.reconn, 0.0, 0.1)
+    x = torch.randn(40, K, device=DEV, dtype=dt, requires_grad=True)
+    dy = torch.randn(40, N, device=DEV, dtype=dt)
+    wanted = [x] + [p for p in layer.parameters() if p.requires_grad]
+    plain = torch.autograd.grad(layer(x), wanted, dy)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: torch.stack((t, -t), -1), lambda s: s[..., 0]):
+        y = layer(x)
+    got = torch.autograd.grad(y, wanted, dy)
+    cp.check_device_status()
+    assert all(torch.equal(a, b) for a, b in zip(plain, got))
+
+
 class _Sub(torch.Tensor):
     pass
 

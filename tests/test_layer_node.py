@@ -1,0 +1,57 @@
+"""The layer's autograd node on the CPU, with the library calls replaced by recorders: what each call is handed."""
+import pytest
+import torch
+
+from cute_mma_b200 import _functional as F
+from cute_mma_b200 import _module
+
+M, K, N, GS, RS = 24, 32, 64, 32, 8
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """Plain eager calls on CPU tensors; the kernels return random numbers and remember their operands."""
+    seen = {}
+
+    def forward(A, B, R, *args, **kw):
+        seen["forward"] = dict(A=A, B=B, R=R, **kw)
+        return torch.zeros(A.shape[0], B.shape[0], dtype=A.dtype), []
+
+    def dadr(dC, A, B, R, *args, internal_bias=None, **kw):
+        seen["dadr"] = dict(dC=dC, A=A, B=B, R=R, internal_bias=internal_bias, **kw)
+        out = torch.randn(A.shape), torch.randn(R.shape)
+        return out if internal_bias is None else out + (torch.randn(internal_bias.shape),)
+
+    def db(dC, A, R, *args, internal_bias=None, **kw):
+        seen["db"] = dict(dC=dC, A=A, R=R, internal_bias=internal_bias, **kw)
+        return torch.randn(dC.shape[1], A.shape[1])
+
+    monkeypatch.setattr(F, "forward", forward)
+    monkeypatch.setattr(F, "_backward_dadr", dadr)
+    monkeypatch.setattr(F, "_backward_db", db)
+    monkeypatch.setattr(F, "bias_grad", lambda dC: dC.sum(0))
+    monkeypatch.setattr(F, "cayley", lambda P, rs: P.clone())
+    monkeypatch.setattr(F, "cayley_backward", lambda P, dP, rs: dP)
+    monkeypatch.setattr(_module, "_plain_eager", lambda *t: True)
+    return seen
+
+
+def _operands():
+    return [torch.randn(*s, requires_grad=True) for s in ((M, K), (N, K), (N // GS * RS, K), (N // GS, K))]
+
+
+def _layer(A, B, R, ib=None, act="silu_gate", cayley=False, seeds=None, p=0.0):
+    return _module._layer_eager(A, B, R, None, ib, seeds, GS, RS, act, 1.0, p, None, cayley)
+
+
+@pytest.mark.parametrize("cayley", [False, True])
+def test_unpacked_tensors_reach_the_kernels_in_rows(calls, cayley):
+    """Saved-tensor hooks may hand back views of another layout: the kernels take whole rows."""
+    A, B, R, ib = _operands()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: torch.stack((t, -t), -1), lambda s: s[..., 0]):
+        y = _layer(A, B, R, None if cayley else ib, "" if cayley else "silu_gate", cayley)
+    y.sum().backward()
+    given = list(calls["dadr"].values()) + list(calls.get("db", {}).values())
+    assert all(t.is_contiguous() for t in given if isinstance(t, torch.Tensor))
+    for name, t in (("A", A), ("B", B), ("R", R)):
+        assert torch.equal(calls["dadr"][name], t.detach())
