@@ -226,17 +226,17 @@ def _plain_eager(*tensors) -> bool:
 
 
 def _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p, fold, cayley):
-    """(C, and the contiguous tensors the kernels were given): P is R, or the Cayley parameter it is made from."""
-    A, weight, P = A.contiguous(), weight.contiguous(), P.contiguous()
+    """(C, and weight, R and internal bias as the backward needs them: the operands themselves, or what was made of
+    them here).  P is R, or the Cayley parameter it is made from."""
     R, rs = P, reconn_sz
     if cayley:
         R = F.cayley(P, reconn_sz)
     if fold is not None:
         weight, R, rs = F.shuffle_cols(weight, fold.inv_seg), F.shuffle_fold_r(R, fold.inv_seg), 64
         ib = None if ib is None else F.shuffle_cols(ib, fold.inv_seg)
-    C, _ = F.forward(A, weight, R, group_size, rs, activation=activation or None, bias=bias, internal_bias=ib,
-                     dropout_p=dropout_p, training=seeds is not None, dropout_seeds=seeds)
-    return C, A, weight, P, R, ib
+    C, _ = F.forward(A.contiguous(), weight.contiguous(), R.contiguous(), group_size, rs, activation=activation or None,
+                     bias=bias, internal_bias=ib, dropout_p=dropout_p, training=seeds is not None, dropout_seeds=seeds)
+    return C, weight, R, ib
 
 
 class _LayerFn(torch.autograd.Function):
@@ -244,8 +244,8 @@ class _LayerFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, cayley):
-        C, A, weight, P, R, ib = _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p,
-                                                fold, cayley)
+        C, weight, R, ib = _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p,
+                                          fold, cayley)
         ctx.save_for_backward(A, weight, R, ib, P if cayley else None)
         ctx.args = group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, bias is not None, seeds
         return C

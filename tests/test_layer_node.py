@@ -55,3 +55,20 @@ def test_unpacked_tensors_reach_the_kernels_in_rows(calls, cayley):
     assert all(t.is_contiguous() for t in given if isinstance(t, torch.Tensor))
     for name, t in (("A", A), ("B", B), ("R", R)):
         assert torch.equal(calls["dadr"][name], t.detach())
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_strided_operands_are_saved_themselves(calls, which):
+    """No copy of a strided operand is kept for the backward, and changing it in between is noticed."""
+    base = [t.detach() for t in _operands()[:3]]
+    base[which] = base[which].t().contiguous().t()
+    ops = [t.requires_grad_() for t in base]
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t.data_ptr()) or t, lambda t: t):
+        _layer(*ops)
+    assert {t.data_ptr() for t in ops} <= set(kept)
+    y = _layer(*ops)
+    with torch.no_grad():
+        ops[which].add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
