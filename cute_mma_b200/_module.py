@@ -63,31 +63,36 @@ def _(A, B, R, bias, group_size, reconn_sz, activation, bwd_scale, internal_bias
     return A.new_empty(A.shape[0], B.shape[0])
 
 
+def _kernel_grads(dC, A, B, R, group_size, reconn_sz, activation, bwd_scale, need_dB, need_dbias, ib, seeds, dropout_p):
+    """(dA, dR, dB, dbias, d_ib) by the kernels, None for what is not asked for.  They take whole rows; saved-tensor
+    hooks may have handed back views of another layout."""
+    dC, A, B, R = dC.contiguous(), A.contiguous(), B.contiguous(), R.contiguous()
+    gate = F._gate_code(activation or None)
+    ib = ib.contiguous() if ib is not None else None
+    mask = F._dropout_mask(seeds if need_dB and gate else None, A.shape[0], B.shape[0], A.shape[1], group_size)
+    out = F._backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
+                           dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
+    dB = None
+    if need_dB and gate:
+        dB = F._backward_db(dC, A, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
+                            dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
+    elif need_dB:
+        dB = torch.zeros_like(B)  # frozen-B contract of the reference's plain mode
+    # the bias is added after the rescale point: its gradient is the plain column sum of dC
+    dbias = F.bias_grad(dC) if need_dbias else None
+    return out[0], out[1], dB, dbias, out[2] if ib is not None else None
+
+
 @torch.library.custom_op("prism_b200::backward", mutates_args=())
 def _prism_backward_op(dC: torch.Tensor, A: torch.Tensor, B: torch.Tensor, R: torch.Tensor,
                        group_size: int, reconn_sz: int, activation: str, bwd_scale: float,
                        need_dB: bool, need_dbias: bool, internal_bias: torch.Tensor | None = None,
                        dropout_seeds: torch.Tensor | None = None, dropout_p: float = 0.0
                        ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
-    dC = dC.contiguous()
-    A, B, R = A.contiguous(), B.contiguous(), R.contiguous()
-    gate = F._gate_code(activation or None)
-    ib = internal_bias.contiguous() if internal_bias is not None else None
-    mask = F._dropout_mask(dropout_seeds if need_dB and gate else None, A.shape[0], B.shape[0], A.shape[1], group_size)
-    out = F._backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
-                           dropout_seeds=dropout_seeds, dropout_p=dropout_p, dropout_mask=mask)
-    dA, dR = out[0], out[1]
-    d_ib = out[2] if ib is not None else dC.new_empty(0)
-    if not need_dB:
-        dB = B.new_empty(0)
-    elif gate:
-        dB = F._backward_db(dC, A, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
-                            dropout_seeds=dropout_seeds, dropout_p=dropout_p, dropout_mask=mask)
-    else:
-        dB = torch.zeros_like(B)  # frozen-B contract of the reference's plain mode
-    # the bias is added after the rescale point: its gradient is the plain column sum of dC
-    dbias = F.bias_grad(dC) if need_dbias else dC.new_empty(0)
-    return dA, dR, dB, dbias, d_ib
+    dA, dR, dB, dbias, d_ib = _kernel_grads(dC, A, B, R, group_size, reconn_sz, activation, bwd_scale, need_dB, need_dbias,
+                                            internal_bias, dropout_seeds, dropout_p)
+    return (dA, dR, B.new_empty(0) if dB is None else dB, dC.new_empty(0) if dbias is None else dbias,
+            dC.new_empty(0) if d_ib is None else d_ib)
 
 
 @_prism_backward_op.register_fake
@@ -225,6 +230,15 @@ def _plain_eager(*tensors) -> bool:
     return True
 
 
+def _plain_grad(dC) -> bool:
+    """Whether an output gradient that passes ``_plain_eager`` is one tensor in memory: not a batch of them
+    (``is_grads_batched``), not the zeros without storage that some formulas hand on."""
+    try:
+        return torch._C._has_storage(dC) and not dC._is_zerotensor()
+    except AttributeError:
+        return False
+
+
 def _layer_forward(A, weight, P, bias, ib, seeds, group_size, reconn_sz, activation, dropout_p, fold, cayley):
     """(C, and weight, R and internal bias as the backward needs them: the operands themselves, or what was made of
     them here).  P is R, or the Cayley parameter it is made from."""
@@ -256,31 +270,19 @@ class _LayerFn(torch.autograd.Function):
         A, weight, R, ib, P = ctx.saved_tensors
         group_size, reconn_sz, activation, bwd_scale, dropout_p, fold, has_bias, seeds = ctx.args
         rs = reconn_sz if fold is None else 64
-        # the kernels take whole rows; saved-tensor hooks may hand back views of another layout
-        dC, A, weight, R = dC.contiguous(), A.contiguous(), weight.contiguous(), R.contiguous()
-        gate = F._gate_code(activation or None)
-        ib = None if ib is None else ib.contiguous()
-        need_dB = ctx.needs_input_grad[1]
-        mask = F._dropout_mask(seeds if need_dB and gate else None, A.shape[0], weight.shape[0], A.shape[1], group_size)
-        out = F._backward_dadr(dC, A, weight, R, group_size, rs, gate, bwd_scale, internal_bias=ib,
-                               dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
-        dA, dP = out[0], out[1]
-        d_ib = out[2] if ib is not None else None
-        dB = None
-        if need_dB:
-            if gate:
-                dB = F._backward_db(dC, A, R, group_size, rs, gate, bwd_scale, internal_bias=ib,
-                                    dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
-            else:
-                dB = torch.zeros_like(weight)  # frozen-B contract of the reference's plain mode
-        # the bias is added after the rescale point: its gradient is the plain column sum of dC
-        dbias = F.bias_grad(dC) if has_bias and ctx.needs_input_grad[3] else None
+        need_dB, need_dbias = ctx.needs_input_grad[1], has_bias and ctx.needs_input_grad[3]
+        # a backward may run under a mode, be traced or be handed a batch of gradients although its forward was ordinary
+        plain = _plain_eager(dC, A, weight, R, ib, P) and _plain_grad(dC)
+        dA, dP, dB, dbias, d_ib = (_kernel_grads if plain else _prism_backward_op)(
+            dC, A, weight, R, group_size, rs, activation, bwd_scale, need_dB, need_dbias, ib, seeds, dropout_p)
+        dB, dbias, d_ib = dB if need_dB else None, dbias if need_dbias else None, None if ib is None else d_ib
         if fold is not None:
-            dP = F.shuffle_unfold_r(dP, fold.perm_seg)
-            dB = None if dB is None else F.shuffle_cols(dB, fold.perm_seg)
-            d_ib = None if d_ib is None else F.shuffle_cols(d_ib, fold.perm_seg)
+            cols = F.shuffle_cols if plain else lambda X, seg: _shuffle_cols_op(X, seg, fold.inv_seg)
+            dP = F.shuffle_unfold_r(dP, fold.perm_seg) if plain else _shuffle_unfold_r_op(dP, fold.perm_seg, fold.inv_seg)
+            dB = None if dB is None else cols(dB, fold.perm_seg)
+            d_ib = None if d_ib is None else cols(d_ib, fold.perm_seg)
         if P is not None and ctx.needs_input_grad[2]:
-            dP = F.cayley_backward(P, dP, reconn_sz)
+            dP = (F.cayley_backward if plain else _cayley_bwd_op)(P, dP, reconn_sz)
         return dA, dB, dP, dbias, d_ib, None, None, None, None, None, None, None, None
 
 

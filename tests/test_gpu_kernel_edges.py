@@ -227,6 +227,30 @@ def test_eager_layer_under_autograd_features():
     cp.check_device_status()
 
 
+@pytest.mark.parametrize("kw", [dict(activation="silu_gate", internal_bias=True), dict(),
+                                dict(activation="silu_gate", input_shuffle=True, reconn_sz=16, internal_bias=True)])
+def test_backward_of_an_ordinary_forward_by_other_means(kw):
+    """A dispatch mode around the backward sees the custom ops; a batch of output gradients is taken one by one: the
+    gradients of the ordinary backward."""
+    K, N, dt = 128, 256, torch.bfloat16
+    torch.manual_seed(3)
+    layer = cp.PrismLinear(K, N, **{"group_size": 64, "reconn_sz": 8, **kw}).to(DEV).to(dt)
+    torch.nn.init.normal_(layer.reconn, 0.0, 0.1)
+    x = torch.randn(40, K, device=DEV, dtype=dt, requires_grad=True)
+    dy = torch.randn(3, 40, N, device=DEV, dtype=dt)
+    wanted = [x] + [p for p in layer.parameters() if p.requires_grad]
+    y = layer(x)
+    plain = [torch.autograd.grad(y, wanted, d, retain_graph=True) for d in dy]
+    mode = _Seen()
+    with mode:
+        seen = torch.autograd.grad(y, wanted, dy[0], retain_graph=True)
+    assert "backward.default" in mode.ops and "forward.default" not in mode.ops
+    batched = torch.autograd.grad(y, wanted, dy, is_grads_batched=True)
+    cp.check_device_status()
+    for i, b in enumerate(batched):
+        assert torch.equal(seen[i], plain[0][i]) and torch.equal(b, torch.stack([p[i] for p in plain]))
+
+
 @pytest.mark.parametrize("kw", [dict(activation="silu_gate", internal_bias=True), dict()])   # the second: Cayley
 def test_unpacked_views_of_another_layout(kw):
     """Saved-tensor hooks that hand back every second element of a wider buffer: the gradients of the plain call."""

@@ -10,28 +10,30 @@ M, K, N, GS, RS = 24, 32, 64, 32, 8
 
 @pytest.fixture
 def calls(monkeypatch):
-    """Plain eager calls on CPU tensors; the kernels return random numbers and remember their operands."""
-    seen = {}
+    """Plain eager calls on CPU tensors; the kernels return made-up numbers and remember their operands."""
+    seen = {"n_dadr": 0}
 
     def forward(A, B, R, *args, **kw):
         seen["forward"] = dict(A=A, B=B, R=R, **kw)
         return torch.zeros(A.shape[0], B.shape[0], dtype=A.dtype), []
 
     def dadr(dC, A, B, R, *args, internal_bias=None, **kw):
+        assert torch._C._has_storage(dC), "a batch of gradients has no address"
         seen["dadr"] = dict(dC=dC, A=A, B=B, R=R, internal_bias=internal_bias, **kw)
-        out = torch.randn(A.shape), torch.randn(R.shape)
-        return out if internal_bias is None else out + (torch.randn(internal_bias.shape),)
+        seen["n_dadr"] += 1
+        out = torch.full(A.shape, float(dC.sum())), torch.ones(R.shape)
+        return out if internal_bias is None else out + (torch.ones(internal_bias.shape),)
 
     def db(dC, A, R, *args, internal_bias=None, **kw):
         seen["db"] = dict(dC=dC, A=A, R=R, internal_bias=internal_bias, **kw)
-        return torch.randn(dC.shape[1], A.shape[1])
+        return torch.ones(dC.shape[1], A.shape[1])
 
     monkeypatch.setattr(F, "forward", forward)
     monkeypatch.setattr(F, "_backward_dadr", dadr)
     monkeypatch.setattr(F, "_backward_db", db)
     monkeypatch.setattr(F, "bias_grad", lambda dC: dC.sum(0))
     monkeypatch.setattr(F, "cayley", lambda P, rs: P.clone())
-    monkeypatch.setattr(F, "cayley_backward", lambda P, dP, rs: dP)
+    monkeypatch.setattr(F, "cayley_backward", lambda P, dP, rs: dP.clone())
     monkeypatch.setattr(_module, "_plain_eager", lambda *t: True)
     return seen
 
@@ -72,3 +74,31 @@ def test_strided_operands_are_saved_themselves(calls, which):
         ops[which].add_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.sum().backward()
+
+
+@pytest.mark.parametrize("cayley", [False, True])
+def test_batched_gradients_are_taken_one_by_one(calls, cayley):
+    """``is_grads_batched`` after an ordinary forward."""
+    A, B, R, ib = _operands()
+    ib, act = (None, "") if cayley else (ib, "silu_gate")
+    wanted = [A, R] if cayley else [A, B, R, ib]
+    dy = torch.randn(3, M, N)
+    got = torch.autograd.grad(_layer(A, B, R, ib, act, cayley), wanted, dy, is_grads_batched=True)
+    assert [g.shape for g in got] == [(3,) + w.shape for w in wanted] and calls["n_dadr"] == 3
+    assert torch.equal(got[0][:, 0, 0], torch.stack([d.sum() for d in dy]))
+
+
+def test_a_mode_around_the_backward_sees_the_custom_ops(calls, monkeypatch):
+    A, B, R, ib = _operands()
+    y = _layer(A, B, R, ib)
+    monkeypatch.setattr(_module, "_plain_eager", lambda *t: False)   # what it answers under a dispatch mode
+    ops = []
+
+    class Seen(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            ops.append(func.namespace + "." + func.__name__)
+            return func(*args, **(kwargs or {}))
+
+    with Seen():
+        torch.autograd.grad(y, A, torch.randn(M, N))
+    assert "prism_b200.backward.default" in ops
