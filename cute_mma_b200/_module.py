@@ -225,7 +225,8 @@ def _plain_eager(*tensors) -> bool:
             or torch.autograd.forward_ad._current_level >= 0):
         return False
     for t in tensors:
-        if t is not None and (type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda):
+        # (a view with the negative bit, as of a conjugate's imaginary part, is in memory what its values are not)
+        if t is not None and (type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda or t.is_neg()):
             return False
     return True
 

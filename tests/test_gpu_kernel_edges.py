@@ -268,6 +268,22 @@ def test_unpacked_views_of_another_layout(kw):
     assert all(torch.equal(a, b) for a, b in zip(plain, got))
 
 
+@pytest.mark.parametrize("grad", [False, True])
+def test_views_with_the_negative_bit(grad):
+    """Values that are the negative of what lies in memory: operands and output gradients alike."""
+    K, N, gs, rs, dt = 128, 256, 64, 8, torch.float16
+    A, B, R, dC = _inputs(40, K, N, gs, rs, dt, 25)
+    A.requires_grad_(grad)
+    y = cp.prism_linear(A, B, R, group_size=gs, reconn_sz=rs, activation="silu_gate")
+    flipped = torch._neg_view(-A)
+    assert flipped.is_neg()
+    assert torch.equal(cp.prism_linear(flipped, B, R, group_size=gs, reconn_sz=rs, activation="silu_gate"), y)
+    if grad:
+        g, = torch.autograd.grad(y, A, dC, retain_graph=True)
+        assert torch.equal(torch.autograd.grad(y, A, torch._neg_view(-dC))[0], g)
+    cp.check_device_status()
+
+
 class _Sub(torch.Tensor):
     pass
 
