@@ -133,8 +133,11 @@ def _cfg_array(cfg):
 
 
 def _raw_stream(device) -> int:
-    """The device's current CUDA stream as a handle, without a Stream object."""
-    return torch._C._cuda_getCurrentRawStream(device.index)
+    """The device's current CUDA stream as a handle; without a Stream object where torch has the private call for it."""
+    try:
+        return torch._C._cuda_getCurrentRawStream(device.index)
+    except AttributeError:
+        return torch.cuda.current_stream(device).cuda_stream
 
 
 class _NoScope:

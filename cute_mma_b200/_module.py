@@ -219,10 +219,13 @@ def _plain_eager(*tensors) -> bool:
     """Whether this call is ordinary eager work on CUDA tensors.  Tracing, compilation, dispatch and function modes, torch.func
     transforms, forward-mode differentiation and tensor subclasses have to see the custom ops, which describe themselves
     to all of these; an ordinary call only pays for that (a custom op costs about 50 us of host time in each direction)."""
-    if (torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
-            or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
-            or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch.autograd.forward_ad._current_level >= 0):
+    try:
+        if (torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
+                or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
+                or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch.autograd.forward_ad._current_level >= 0):
+            return False
+    except AttributeError:   # private names: in a torch that has lost one, every call runs the custom ops
         return False
     for t in tensors:
         # (a view with the negative bit, as of a conjugate's imaginary part, is in memory what its values are not)

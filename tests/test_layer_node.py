@@ -102,3 +102,24 @@ def test_a_mode_around_the_backward_sees_the_custom_ops(calls, monkeypatch):
     with Seen():
         torch.autograd.grad(y, A, torch.randn(M, N))
     assert "prism_b200.backward.default" in ops
+
+
+class _OnGpu(torch.Tensor):
+    is_cuda = True
+
+
+@pytest.mark.parametrize("owner,name", [(torch._C, "_get_tracing_state"), (torch._C, "_len_torch_dispatch_stack"),
+                                        (torch._C, "_len_torch_function_stack"), (torch._C._functorch, "peek_interpreter_stack"),
+                                        (torch.autograd.forward_ad, "_current_level")])
+def test_a_torch_without_a_private_name_runs_the_custom_ops(monkeypatch, owner, name):
+    t = torch.zeros(2).as_subclass(_OnGpu)
+    monkeypatch.setattr(torch, "Tensor", _OnGpu)   # so that an ordinary call is one on this machine's tensors
+    assert _module._plain_eager(t)
+    monkeypatch.delattr(owner, name)
+    assert not _module._plain_eager(t)
+
+
+def test_a_torch_without_the_raw_stream_call(monkeypatch):
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: type("Stream", (), {"cuda_stream": 77}))
+    assert F._raw_stream(torch.device("cuda", 0)) == 77
