@@ -419,12 +419,47 @@ def shuffle_unfold_r(dR64, perm_seg):
 _MASK_BYTES_MAX = 1 << 30   # beyond this the dB kernel hashes again instead
 
 
-def _dropout_mask(seeds, M, N, K, group_size):
-    """Scratch in which the dA+dR kernel leaves the dropout mask for the dB kernel of the same backward, or None."""
-    if seeds is None:
+def _dropout_mask(seeds, p, M, N, K, group_size):
+    """Scratch in which the dA+dR kernel leaves the dropout mask for the dB kernel of the same backward, or None: without
+    dropout, and where the scratch is too large or there is no memory for it."""
+    if seeds is None or not p > 0.0:
         return None
     nbytes = _lib.lib().prism_dropout_mask_bytes(M, N, K, group_size)
-    return torch.empty(nbytes // 4, dtype=torch.int32, device=seeds.device) if 0 < nbytes <= _MASK_BYTES_MAX else None
+    if not 0 < nbytes <= _MASK_BYTES_MAX:
+        return None
+    try:
+        return torch.empty(nbytes // 4, dtype=torch.int32, device=seeds.device)
+    except torch.OutOfMemoryError:
+        return None
+
+
+def _backward_both(dC, A, B, R, group_size, reconn_sz, gate, dc_scale=1.0, need_dB=True, internal_bias=None, seeds=None,
+                   dropout_p=0.0, tile_cfg_dadr=None, tile_cfg_db=None, dR_dtype=None, dB_dtype=None):
+    """(dA, dR, dB, d_internal_bias) by the dA+dR kernel and, in the gated modes where dB is wanted, the dB kernel; None for
+    what there is none of.  The dropout mask that the first leaves for the second is only an economy: where its memory
+    is needed for anything else of the two calls, it is given back and the dB kernel hashes for itself."""
+    need_dB = need_dB and gate != 0
+    mask = _dropout_mask(seeds, dropout_p, A.shape[0], B.shape[0], A.shape[1], group_size) if need_dB else None
+
+    def without_mask_if_short(call):
+        nonlocal mask
+        try:
+            return call(mask)
+        except torch.OutOfMemoryError:
+            if mask is None:
+                raise
+        mask = None   # out here, where the failed call's frames are gone and with them their references to it
+        return call(None)
+
+    out = without_mask_if_short(lambda m: _backward_dadr(
+        dC, A, B, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_dadr, dR_dtype, internal_bias=internal_bias,
+        dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=m))
+    dB = None
+    if need_dB:
+        dB = without_mask_if_short(lambda m: _backward_db(
+            dC, A, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_db, dB_dtype, internal_bias=internal_bias,
+            dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=m))
+    return out[0], out[1], dB, out[2] if internal_bias is not None else None
 
 
 def _out_buffer(out, shape, dtype, device, name):
@@ -530,12 +565,8 @@ def backward(dC, A, B, R, group_size: int = 256, reconn_sz: int = 8, backend=Non
     if gate and dropout_seeds is not None and dropout_p > 0.0:
         _check_dropout(dropout_p, reconn_sz)
         seeds = _check_seeds(dropout_seeds, A, N // group_size)
-    mask = _dropout_mask(seeds, M, N, K, group_size)
-    out = _backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_dadr, dR_dtype, internal_bias,
-                         seeds, dropout_p, dropout_mask=mask)
-    dB = (_backward_db(dC, A, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_db, dB_dtype, internal_bias,
-                       seeds, dropout_p, dropout_mask=mask) if gate else None)
-    return out[0], out[1], dB, (out[2] if internal_bias is not None else None)
+    return _backward_both(dC, A, B, R, group_size, reconn_sz, gate, dc_scale, True, internal_bias, seeds, dropout_p,
+                          tile_cfg_dadr, tile_cfg_db, dR_dtype, dB_dtype)
 
 
 def bias_grad(dC, out_dtype=None):

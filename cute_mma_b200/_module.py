@@ -69,18 +69,12 @@ def _kernel_grads(dC, A, B, R, group_size, reconn_sz, activation, bwd_scale, nee
     dC, A, B, R = dC.contiguous(), A.contiguous(), B.contiguous(), R.contiguous()
     gate = F._gate_code(activation or None)
     ib = ib.contiguous() if ib is not None else None
-    mask = F._dropout_mask(seeds if need_dB and gate else None, A.shape[0], B.shape[0], A.shape[1], group_size)
-    out = F._backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
-                           dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
-    dB = None
-    if need_dB and gate:
-        dB = F._backward_db(dC, A, R, group_size, reconn_sz, gate, bwd_scale, internal_bias=ib,
-                            dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=mask)
-    elif need_dB:
+    dA, dR, dB, d_ib = F._backward_both(dC, A, B, R, group_size, reconn_sz, gate, bwd_scale, need_dB, ib, seeds, dropout_p)
+    if need_dB and not gate:
         dB = torch.zeros_like(B)  # frozen-B contract of the reference's plain mode
     # the bias is added after the rescale point: its gradient is the plain column sum of dC
     dbias = F.bias_grad(dC) if need_dbias else None
-    return out[0], out[1], dB, dbias, out[2] if ib is not None else None
+    return dA, dR, dB, dbias, d_ib
 
 
 @torch.library.custom_op("prism_b200::backward", mutates_args=())

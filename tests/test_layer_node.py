@@ -123,3 +123,56 @@ def test_a_torch_without_the_raw_stream_call(monkeypatch):
     monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device: type("Stream", (), {"cuda_stream": 77}))
     assert F._raw_stream(torch.device("cuda", 0)) == 77
+
+
+@pytest.mark.parametrize("short", ["mask", "dadr", "db", "both", "always"])
+@pytest.mark.parametrize("call", ["layer", "op", "backward"])
+def test_backward_with_dropout_where_memory_is_short(calls, built_lib, monkeypatch, short, call):
+    """The mask handed from dA+dR to dB is given up where it, or what else the calls need beside it, does not fit; a call
+    that does not fit without it fails as before."""
+    import weakref
+    A, B, R, ib = _operands()
+    seeds, masks, given = torch.arange(1, N // GS + 1), [], []
+    empty = torch.empty
+
+    def mask_or_not(*shape, **kw):
+        if kw.get("dtype") != torch.int32:
+            return empty(*shape, **kw)
+        if short == "mask":
+            raise torch.OutOfMemoryError("no memory")
+        t = empty(*shape, **kw)
+        masks.append(weakref.ref(t))
+        return t
+
+    def needs(name, kernel):
+        def f(*args, dropout_mask=None, **kw):
+            given.append((name, dropout_mask is not None))
+            alive = any(m() is not None for m in masks)
+            assert alive == (dropout_mask is not None), "a mask given up is a mask freed"
+            if short == "always" or (alive and short in (name, "both")):
+                raise torch.OutOfMemoryError("no memory")
+            return kernel(*args, **kw)
+        return f
+
+    monkeypatch.setattr(torch, "empty", mask_or_not)
+    monkeypatch.setattr(F, "_backward_dadr", needs("dadr", F._backward_dadr))
+    monkeypatch.setattr(F, "_backward_db", needs("db", F._backward_db))
+    if call == "backward":
+        monkeypatch.setattr(F, "validate_tensor_params", lambda *a: None)
+        run = lambda: F.backward(torch.ones(M, N), A.detach(), B.detach(), R.detach(), GS, RS, activation="silu_gate",   # noqa: E731
+                                 dropout_seeds=seeds, dropout_p=0.5)
+    elif call == "op":
+        run = lambda: _module._prism_backward_op(torch.ones(M, N), A.detach(), B.detach(), R.detach(), GS, RS,   # noqa: E731
+                                                 "silu_gate", 1.0, True, False, None, seeds, 0.5)
+    else:
+        run = lambda: _layer(A, B, R, ib, seeds=seeds, p=0.5).sum().backward()   # noqa: E731
+    if short == "always":
+        with pytest.raises(torch.OutOfMemoryError):
+            run()
+        return
+    run()
+    with_mask, without = True, False
+    assert given == {"mask": [("dadr", without), ("db", without)],
+                     "dadr": [("dadr", with_mask), ("dadr", without), ("db", without)],
+                     "both": [("dadr", with_mask), ("dadr", without), ("db", without)],
+                     "db": [("dadr", with_mask), ("db", with_mask), ("db", without)]}[short]
