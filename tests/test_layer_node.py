@@ -176,3 +176,17 @@ def test_backward_with_dropout_where_memory_is_short(calls, built_lib, monkeypat
                      "dadr": [("dadr", with_mask), ("dadr", without), ("db", without)],
                      "both": [("dadr", with_mask), ("dadr", without), ("db", without)],
                      "db": [("dadr", with_mask), ("db", with_mask), ("db", without)]}[short]
+
+
+@pytest.mark.parametrize("op", [False, True])
+def test_dropout_seeds_reach_the_kernels_as_the_forward_took_them(calls, monkeypatch, op):
+    """Seeds given as every second element of a tensor (or on another device): the kernels read them one after the other."""
+    A, B, R, ib = _operands()
+    seeds = torch.arange(1, 2 * (N // GS) + 1)[::2]
+    y = _layer(A, B, R, ib, seeds=seeds, p=0.5)
+    if op:
+        monkeypatch.setattr(_module, "_plain_eager", lambda *t: False)
+    y.sum().backward()
+    for name in ("dadr", "db"):
+        given = calls[name]["dropout_seeds"]
+        assert given.is_contiguous() and given.device == A.device and torch.equal(given, seeds)
