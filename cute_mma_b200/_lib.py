@@ -33,7 +33,7 @@ EXPORTS = [
     "prism_last_error_string", "prism_abi_version", "prism_launch_count",
 ]
 
-ABI_VERSION = 4
+ABI_VERSION = 5   # prism_abi_version() of a library that has all of EXPORTS
 
 _lock = threading.Lock()
 _lib = None
@@ -108,6 +108,11 @@ def lib() -> ctypes.CDLL:
                     "or cute_mma_b200._lib.build(); there is no fallback path")
             L = ctypes.CDLL(LIB_PATH)
             vp, ll, i, sz = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_size_t
+            # first of all: a library of another version may lack the symbols bound below
+            L.prism_abi_version.restype = i
+            if L.prism_abi_version() != ABI_VERSION:
+                raise RuntimeError(f"{LIB_PATH} has ABI version {L.prism_abi_version()}, this package needs "
+                                   f"{ABI_VERSION}: rebuild it (cute_mma_b200._lib.build(force=True))")
             ip = ctypes.POINTER(ctypes.c_int)
             L.prism_fwd.restype = i
             L.prism_fwd.argtypes = [vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, ll, ll, ll, ll, ip, vp, sz, vp]
@@ -154,10 +159,6 @@ def lib() -> ctypes.CDLL:
             L.prism_status.argtypes = [vp, vp]
             L.prism_last_error_string.restype = ctypes.c_char_p
             L.prism_last_error_string.argtypes = []
-            L.prism_abi_version.restype = i
-            if L.prism_abi_version() != ABI_VERSION:
-                raise RuntimeError(f"{LIB_PATH} has ABI version {L.prism_abi_version()}, this package needs "
-                                   f"{ABI_VERSION}: rebuild it (cute_mma_b200._lib.build(force=True))")
             L.prism_launch_count.restype = ll
             _lib = L
         return _lib

@@ -250,7 +250,7 @@ static int check_ptr(const char* fn, const char* name, const void* p, long long 
 
 using namespace prism;
 
-extern "C" int prism_abi_version(void) { return 4; }
+extern "C" int prism_abi_version(void) { return 5; }
 
 extern "C" long long prism_launch_count(void) { return launch_counter().load(std::memory_order_relaxed); }
 

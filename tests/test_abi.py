@@ -24,7 +24,19 @@ def test_header_and_loader_agree():
 def test_library_exports_every_declared_symbol(built_lib):
     for name in _declared_symbols():
         assert hasattr(built_lib, name), name
-    assert built_lib.prism_abi_version() == _lib.ABI_VERSION == 4
+    assert built_lib.prism_abi_version() == _lib.ABI_VERSION == 5
+
+
+def test_a_library_of_another_version_is_named_as_such(tmp_path, monkeypatch):
+    """Before anything it may lack is looked up: version 4 had none of the dropout-mask and shuffle functions."""
+    import subprocess
+    src, so = tmp_path / "old.c", tmp_path / "libold.so"
+    src.write_text("int prism_abi_version(void) { return 4; }")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(so), str(src)], check=True)
+    monkeypatch.setattr(_lib, "LIB_PATH", str(so))
+    monkeypatch.setattr(_lib, "_lib", None)
+    with pytest.raises(RuntimeError, match="ABI version 4, this package needs 5: rebuild it"):
+        _lib.lib()
 
 
 def _call_fwd(L, M, N, K, gs, rs, dtype=1, gate=0, ptr=0x1000, ws=0x1000, ws_bytes=1 << 20):
