@@ -79,7 +79,8 @@ struct DbBarriers {
   uint32_t tmem_base;
 };
 
-template <int DT, int GATE, int E, bool DROP>
+// WIDEN: reconn_sz 8, R is widened here (E = 16); an instance of its own (see prism_fwd_small.cu)
+template <int DT, int GATE, int E, bool DROP, bool WIDEN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(db::kThreads, 1)
 prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmR,
                     const __grid_constant__ CUtensorMap tmdC, const __grid_constant__ CUtensorMap tmdB, const DbParams p) {
@@ -116,7 +117,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
   }
-  if (E == 16 && p.R8 != nullptr && threadIdx.x < 256) {
+  if (WIDEN && threadIdx.x < 256) {
     // Two tiles of 16 rows x 8 pieces (8 features): row i of the widened block holds R's row i % 8 in the pieces of parity
     // i / 8.  A launch of its own for this copy cost 2 to 3 us before every call.
     const int t = threadIdx.x >> 7, i = (threadIdx.x >> 3) & 15, c = threadIdx.x & 7;
@@ -148,7 +149,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       bool ok = true;
-      if (E != 16 || p.R8 == nullptr) {
+      if (!WIDEN) {
         mbar_arrive_expect_tx(&bars->r_full, 2 * E * 128);
         tma_load_2d(smemR, &tmR, &bars->r_full, f0, g * E);
         tma_load_2d(smemR + p.r_tile_bytes, &tmR, &bars->r_full, f0 + 64, g * E);
@@ -450,14 +451,18 @@ int launch_bwd_db(const DbArgs& a) {
 
   using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, DbParams);
   KernT kern = nullptr;
-#define PRISM_PICK_G(DT_, E_, DROP_)                                                                    \
-  (a.gate == GATE_SILU ? (KernT)prism_bwd_db_kernel<DT_, GATE_SILU, E_, DROP_>                           \
-                       : a.gate == GATE_SIGMOID ? (KernT)prism_bwd_db_kernel<DT_, GATE_SIGMOID, E_, DROP_> : (KernT)prism_bwd_db_kernel<DT_, GATE_NONE, E_, false>)
-#define PRISM_PICK(E_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_G(DT_BF16, E_, false) : PRISM_PICK_G(DT_F16, E_, false)
-  if (drop) { kern = (a.dtype == DT_BF16) ? PRISM_PICK_G(DT_BF16, 16, true) : PRISM_PICK_G(DT_F16, 16, true); }
-  else if (a.E == 16) { PRISM_PICK(16); } else if (a.E == 32) { PRISM_PICK(32); } else { PRISM_PICK(64); }
+#define PRISM_PICK_W(DT_, E_, DROP_, W_)                                                                 \
+  (a.gate == GATE_SILU ? (KernT)prism_bwd_db_kernel<DT_, GATE_SILU, E_, DROP_, W_>                        \
+                       : a.gate == GATE_SIGMOID ? (KernT)prism_bwd_db_kernel<DT_, GATE_SIGMOID, E_, DROP_, W_> \
+                                                : (KernT)prism_bwd_db_kernel<DT_, GATE_NONE, E_, false, W_>)
+#define PRISM_PICK_G(E_, DROP_, W_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_W(DT_BF16, E_, DROP_, W_) : PRISM_PICK_W(DT_F16, E_, DROP_, W_)
+#define PRISM_PICK_16(DROP_) if (a.widen) { PRISM_PICK_G(16, DROP_, true); } else { PRISM_PICK_G(16, DROP_, false); }
+  if (drop) { PRISM_PICK_16(true) }
+  else if (a.E == 16) { PRISM_PICK_16(false) }
+  else if (a.E == 32) { PRISM_PICK_G(32, false, false); } else { PRISM_PICK_G(64, false, false); }
+#undef PRISM_PICK_16
+#undef PRISM_PICK_W
 #undef PRISM_PICK_G
-#undef PRISM_PICK
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_db"))) return rc;
   const int rows = a.N / a.BN;
   // one launch over the n-tile rows [nt0, nt0 + nrows) with the token range of every tile split `splits` ways

@@ -127,7 +127,8 @@ __device__ __forceinline__ void epilogue_cols32(uint32_t tacc, uint8_t* stage, i
 }
 
 // EXTRA: 0 the plain gate warps; 1 internal bias (a null bias is allowed); 2 hash dropout (+ optional bias)
-template <int DT, int GATE, int E, int EXTRA>
+// WIDEN: reconn_sz 8 in a short call, R is widened here (E = 16); an instance of its own, so that the others stay as they are
+template <int DT, int GATE, int E, int EXTRA, bool WIDEN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(fwd::kThreads, 1)
 prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmR,
                  const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
@@ -155,7 +156,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxStages; ++i) {
       // two producers in each CTA, one arrive.expect_tx each (and one arrive for a R tile written by warp 0)
-      mbar_init(&bars->loads_full[i], (E == 16 && p.R8 != nullptr) ? 6 : 4);
+      mbar_init(&bars->loads_full[i], WIDEN ? 6 : 4);
       mbar_init(&bars->done[i], 1);
     }
     for (int i = 0; i < kSlots; ++i) {
@@ -166,7 +167,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     mbar_init(&bars->acc_empty, 2 * kNumEpiWarps);
     fence_mbar_init();
   }
-  if (E == 16 && p.R8 != nullptr) {
+  if (WIDEN) {
     // the blocks off the widened diagonal stay zero for good: the producer only writes the others
     for (int i = threadIdx.x; i < p.ns * 64; i += kThreads)
       *reinterpret_cast<uint4*>(smemSt + (i >> 6) * p.stage_bytes + kATileBytes + (i & 63) * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -193,7 +194,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int my_tiles = (p.n_tiles - cid + n_clusters - 1) / n_clusters;
   const uint32_t total = (uint32_t)my_tiles * nk;   // chunks this CTA pair processes
 
-  if (E == 16 && warp == kWarpTma && p.R8 != nullptr) {
+  if (WIDEN && warp == kWarpTma) {
     // ------------------------------------------------------------------ producer for reconn_sz 8: A tile by TMA, R by hand
     // This CTA's eight rows of the widened R tile are R's eight rows of the group in every second piece of 8 features
     // (the leader the even ones, the peer the odd ones): one 16-byte piece per lane, fetched a chunk ahead.  For
@@ -534,14 +535,19 @@ int launch_fwd(const FwdArgs& a) {
 
   using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdParams);
   KernT kern = nullptr;
-#define PRISM_PICK_G(DT_, E_, X_)                                                                       \
-  (a.gate == GATE_SILU ? (KernT)prism_fwd_kernel<DT_, GATE_SILU, E_, X_>                                 \
-                       : a.gate == GATE_SIGMOID ? (KernT)prism_fwd_kernel<DT_, GATE_SIGMOID, E_, X_> : (KernT)prism_fwd_kernel<DT_, GATE_NONE, E_, 0>)
-#define PRISM_PICK(E_, X_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_G(DT_BF16, E_, X_) : PRISM_PICK_G(DT_F16, E_, X_)
+#define PRISM_PICK_W(DT_, E_, X_, W_)                                                                    \
+  (a.gate == GATE_SILU ? (KernT)prism_fwd_kernel<DT_, GATE_SILU, E_, X_, W_>                              \
+                       : a.gate == GATE_SIGMOID ? (KernT)prism_fwd_kernel<DT_, GATE_SIGMOID, E_, X_, W_>  \
+                                                : (KernT)prism_fwd_kernel<DT_, GATE_NONE, E_, 0, W_>)
+#define PRISM_PICK_G(E_, X_, W_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_W(DT_BF16, E_, X_, W_) : PRISM_PICK_W(DT_F16, E_, X_, W_)
+#define PRISM_PICK(X_)                                                                                   \
+  if (a.widen) { PRISM_PICK_G(16, X_, true); } else if (a.E == 16) { PRISM_PICK_G(16, X_, false); }       \
+  else if (a.E == 32) { PRISM_PICK_G(32, X_, false); } else { PRISM_PICK_G(64, X_, false); }
   const bool ib = a.ib != nullptr && a.gate != GATE_NONE;
-  if (drop) { PRISM_PICK(16, 2); }
-  else if (ib) { if (a.E == 16) { PRISM_PICK(16, 1); } else if (a.E == 32) { PRISM_PICK(32, 1); } else { PRISM_PICK(64, 1); } }
-  else if (a.E == 16) { PRISM_PICK(16, 0); } else if (a.E == 32) { PRISM_PICK(32, 0); } else { PRISM_PICK(64, 0); }
+  if (drop) { if (a.widen) { PRISM_PICK_G(16, 2, true); } else { PRISM_PICK_G(16, 2, false); } }
+  else if (ib) { PRISM_PICK(1) }
+  else { PRISM_PICK(0) }
+#undef PRISM_PICK_W
 #undef PRISM_PICK_G
 #undef PRISM_PICK
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "forward"))) return rc;

@@ -48,7 +48,7 @@ struct FwdSmallParams {
   int units, ncta;     // G * nk work units over ncta CTAs
   int pmax;            // partial slots per group
   int ns, stage_bytes, a_off, r_off, b_off;
-  const uint16_t* R8;  // reconn_sz 8: R [G*8, K] itself, or null: the R tiles come through tmR
+  const uint16_t* R8;  // reconn_sz 8: R [G*8, K] itself, else null: the R tiles come through tmR
   long long ldr;
   const void* bias;
   const void* ib;      // internal bias [G, K] or null
@@ -77,7 +77,9 @@ __device__ __host__ __forceinline__ int fsm_owner(long long x, int units, int nc
   return (int)(((x + 1) * ncta + units - 1) / units) - 1;
 }
 
-template <int DT, int GATE, int E, bool DROP>
+// WIDEN: reconn_sz 8, R is widened here (E = 16).  An instance of its own: with the choice made at run time, the instance for
+// reconn_sz 16 took 0.3 us longer a call (1 token, 1024 -> 4096: 9.8 / 10.2 us).
+template <int DT, int GATE, int E, bool DROP, bool WIDEN>
 __global__ void __launch_bounds__(fsm::kThreads, 1)
 prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmR,
                        const __grid_constant__ CUtensorMap tmB, const FwdSmallParams p) {
@@ -120,7 +122,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmR);
   }
-  if (E == 16 && p.R8 != nullptr) {
+  if (WIDEN) {
     // the blocks off the widened diagonal stay zero for good: the rotation's warp only writes the others
     for (int i = threadIdx.x; i < p.ns * 128; i += kThreads)
       *reinterpret_cast<uint4*>(smemSt + (i >> 7) * p.stage_bytes + p.r_off + (i & 127) * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -133,8 +135,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   // the producer fills the ring's first pass before the CTA-wide synchronisation: nothing else has
   // touched these stages yet, so their "empty" barriers need no wait
   const uint64_t pol = l2_policy_evict_first();
-  const bool widen = E == 16 && p.R8 != nullptr;   // reconn_sz 8: the rotation's warp writes the R tile
-  const uint32_t stage_tx = (uint32_t)(p.nrt * kTile + p.Mp * 128 + (widen ? 0 : E * 128));
+  const uint32_t stage_tx = (uint32_t)(p.nrt * kTile + p.Mp * 128 + (WIDEN ? 0 : E * 128));   // WIDEN: the rotation's warp writes the R tile
   int pre = 0;
   if (threadIdx.x == 0) {
     int g = u0 / p.nk, kc = u0 - g * p.nk;
@@ -144,7 +145,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       for (int j = 0; j < p.nrt; ++j)
         tma_load_2d_hint(dst + p.b_off + j * kTile, &tmB, &bars->full[pre], kc * 64, g * p.gs + j * 128, pol);
       tma_load_2d(dst + p.a_off, &tmA, &bars->full[pre], kc * 64, 0);
-      if (!widen) tma_load_2d(dst + p.r_off, &tmR, &bars->full[pre], kc * 64, g * E);
+      if (!WIDEN) tma_load_2d(dst + p.r_off, &tmR, &bars->full[pre], kc * 64, g * E);
       if (++kc == p.nk) { kc = 0; ++g; }
     }
   }
@@ -170,7 +171,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         for (int j = 0; j < p.nrt; ++j)
           tma_load_2d_hint(dst + p.b_off + j * kTile, &tmB, &bars->full[rs.idx], kc * 64, g * p.gs + j * 128, pol);
         tma_load_2d(dst + p.a_off, &tmA, &bars->full[rs.idx], kc * 64, 0);
-        if (!widen) tma_load_2d(dst + p.r_off, &tmR, &bars->full[rs.idx], kc * 64, g * E);
+        if (!WIDEN) tma_load_2d(dst + p.r_off, &tmR, &bars->full[rs.idx], kc * 64, g * E);
         if (++kc == p.nk) { kc = 0; ++g; }
       }
       if (!ok) atomicExch(p.err, PRISM_ERR_DEVICE_WAIT);
@@ -180,7 +181,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // reconn_sz 8: the warp first writes the unit's R tile, two 8 x 8 blocks of R widened to one of 16 x 16.  Row i of the
     // widened blocks is R's row i % 8 in the pieces of 8 features of parity i / 8: two 16-byte pieces per lane, fetched a
     // unit ahead.  (A launch of its own for the widened copy: 2.2 us of 19 for 20 tokens, 1024 -> 16384.)
-    if (lane == 0 || widen) {
+    if (WIDEN || lane == 0) {
       const int r_row = lane >> 2, r_piece = (lane & 3) * 2;   // and row + 8, piece + 1
       int gr = u0 / p.nk, kr = u0 - gr * p.nk;
       uint4 r_even = make_uint4(0u, 0u, 0u, 0u), r_odd = r_even;
@@ -191,7 +192,7 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         r_odd = col + 8 < p.K ? __ldg(reinterpret_cast<const uint4*>(src) + 1) : make_uint4(0u, 0u, 0u, 0u);
         if (++kr == p.nk) { kr = 0; ++gr; }
       };
-      if (widen && u0 < u1) fetch();
+      if (WIDEN && u0 < u1) fetch();
       const uint32_t idesc_r = make_idesc(DT, 128, E, 0, 0);        // S block: M = 128 token rows, N = E
       const uint64_t d0 = desc_kmajor_sw128(smem_u32(smemSt), 1024);
       const uint32_t d_hi = (uint32_t)(d0 >> 32);
@@ -204,11 +205,11 @@ prism_fwd_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         const uint32_t slot = (uint32_t)i & 1u;
         if (i >= 2) {   // the gate warps hold S of unit i - 2 in registers
           const bool got = mbar_wait(&bars->s_free[slot], (((uint32_t)i >> 1) - 1) & 1);
-          if (widen ? !__all_sync(0xffffffffu, got) : !got) { ok = false; break; }
+          if (WIDEN ? !__all_sync(0xffffffffu, got) : !got) { ok = false; break; }
         }
         const bool got = mbar_wait(&bars->full[rl.idx], rl.phase);
-        if (widen ? !__all_sync(0xffffffffu, got) : !got) { ok = false; break; }
-        if (widen) {   // the stage is this unit's, the rotation that read its R tile before has long completed
+        if (WIDEN ? !__all_sync(0xffffffffu, got) : !got) { ok = false; break; }
+        if (WIDEN) {   // the stage is this unit's, the rotation that read its R tile before has long completed
           uint8_t* rt = smemSt + rl.idx * p.stage_bytes + p.r_off;
           *reinterpret_cast<uint4*>(rt + sw128_offset(r_row, r_piece)) = r_even;
           *reinterpret_cast<uint4*>(rt + sw128_offset(r_row + 8, r_piece + 1)) = r_odd;
@@ -439,14 +440,18 @@ int launch_fwd_small(const FwdArgs& a, void* scratch) {
 
   using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FwdSmallParams);
   KernT kern = nullptr;
-#define PRISM_PICK_G(DT_, E_, DROP_)                                                                    \
-  (a.gate == GATE_SILU ? (KernT)prism_fwd_small_kernel<DT_, GATE_SILU, E_, DROP_>                        \
-                       : a.gate == GATE_SIGMOID ? (KernT)prism_fwd_small_kernel<DT_, GATE_SIGMOID, E_, DROP_> : (KernT)prism_fwd_small_kernel<DT_, GATE_NONE, E_, false>)
-#define PRISM_PICK(E_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_G(DT_BF16, E_, false) : PRISM_PICK_G(DT_F16, E_, false)
-  if (drop) { kern = (a.dtype == DT_BF16) ? PRISM_PICK_G(DT_BF16, 16, true) : PRISM_PICK_G(DT_F16, 16, true); }
-  else if (a.E == 16) { PRISM_PICK(16); } else if (a.E == 32) { PRISM_PICK(32); } else { PRISM_PICK(64); }
+#define PRISM_PICK_W(DT_, E_, DROP_, W_)                                                                 \
+  (a.gate == GATE_SILU ? (KernT)prism_fwd_small_kernel<DT_, GATE_SILU, E_, DROP_, W_>                     \
+                       : a.gate == GATE_SIGMOID ? (KernT)prism_fwd_small_kernel<DT_, GATE_SIGMOID, E_, DROP_, W_> \
+                                                : (KernT)prism_fwd_small_kernel<DT_, GATE_NONE, E_, false, W_>)
+#define PRISM_PICK_G(E_, DROP_, W_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_W(DT_BF16, E_, DROP_, W_) : PRISM_PICK_W(DT_F16, E_, DROP_, W_)
+#define PRISM_PICK_16(DROP_) if (a.widen) { PRISM_PICK_G(16, DROP_, true); } else { PRISM_PICK_G(16, DROP_, false); }
+  if (drop) { PRISM_PICK_16(true) }
+  else if (a.E == 16) { PRISM_PICK_16(false) }
+  else if (a.E == 32) { PRISM_PICK_G(32, false, false); } else { PRISM_PICK_G(64, false, false); }
+#undef PRISM_PICK_16
+#undef PRISM_PICK_W
 #undef PRISM_PICK_G
-#undef PRISM_PICK
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "small-M forward"))) return rc;
   kern<<<p.ncta, fsm::kThreads, smem_bytes, a.stream>>>(tmA, tmR, tmB, p);
   if ((rc = check_launch("prism_fwd_small"))) return rc;
