@@ -3,6 +3,7 @@
 #include "../../include/prism_b200.h"
 #include "prism_host.cuh"
 #include "prism_kernels.cuh"
+#include "prism_plan.h"
 
 namespace prism {
 
@@ -160,36 +161,6 @@ static int effective_block(int rs) {
   if (rs == 8) return 16;
   if (rs == 16 || rs == 32 || rs == 64) return rs;
   return 0;
-}
-
-// Widest n-tile of a group: the largest multiple of 32 up to 256 that divides group_size, or 16.  A narrow tile reloads
-// A and repeats the rotation and the gate for every tile of the group.
-// Measured against the powers of two used before, 2000 x 3000 -> 6144 with groups of 192 (64 -> 192 wide): forward 218 ->
-// 92 us, dB 323 -> 134 us; 1000 x 1000 -> 1440 with groups of 96 (32 -> 96): 31 -> 17 and 40 -> 16 us.  Widths that are
-// multiples of 16 only are left at 16.
-static int default_bn(int gs) {
-  for (int c = 256; c >= 32; c -= 32)
-    if (gs % c == 0) return c;
-  return gs % 16 == 0 ? 16 : 0;
-}
-
-// n-tile of the general forward: the widest, halved (down to 64) as long as the narrower tiles still run in one wave.  A
-// narrow tile repeats its group's rotation and gate, but on a CTA pair that would be idle, and its epilogue is shorter.
-// Measured, 256 against 64 wide: 1024 x 256 -> 1024 8.9 / 7.1 us, 1024 x 768 -> 768 12.8 / 10.7; 200 x 4096 -> 1024 32.6 /
-// 30.4; 32 wide is no faster (8.8, 15.7, 30.3), and two waves lose (128 x 4096 -> 14336: 36.7 / 104.9).
-static int fwd_default_bn(int M, int N, int gs, int sms) {
-  int bn = default_bn(gs);
-  while (bn % 64 == 0 && bn >= 128 && (long long)((M + 255) / 256) * (N / (bn / 2)) <= sms / 2) bn /= 2;
-  return bn;
-}
-
-// Whether the general forward widens rotations of 8 itself or gets a widened copy of R from a launch before it (about 2 us,
-// and its host time): itself where a CTA pair has few chunks of 64 features to go through.  Measured, copy against
-// itself: 4 chunks 10.3 -> 9.1 us, 12 chunks 12.7 -> 11.9, 16 chunks 14.5 -> 13.9; 132 chunks (plain mode) 80 -> 78-81;
-// 448 chunks 269 -> 318, 448 of a deeper layer 228 -> 303.
-static bool fwd_widens(int M, int N, int K, int bn, int sms) {
-  const long long tiles = (long long)((M + 255) / 256) * (N / bn), pairs = sms / 2 > 0 ? sms / 2 : 1;
-  return (tiles + pairs - 1) / pairs * ((K + 63) / 64) <= 32;
 }
 
 static int check_common(const char* fn, int M, int N, int K, int gs, int rs, int dtype, int gate) {
@@ -379,7 +350,7 @@ extern "C" int prism_fwd_dropout(const void* A, const void* B, const void* R, co
     return fail(PRISM_ERR_UNSUPPORTED, "%s: the few-token kernel needs M <= 128 and group_size a multiple of 128 (M=%d, group_size=%d)", fn, M, gs);
   if (path != 1 && fwd_small_supported(M, N, K, gs, a.E) && (path == 2 || fwd_small_preferred(M)))
     return launch_fwd_small(a, wp);
-  a.BN = (cfg && cfg[0] > 0) ? cfg[0] : fwd_default_bn(M, N, gs, a.num_sms);
+  a.BN = (cfg && cfg[0] > 0) ? cfg[0] : fwd_default_bn(M, N, K, gs, bias != nullptr, a.num_sms);
   a.PM = (cfg && cfg[1] > 0) ? cfg[1] : 16;
   a.sa = (cfg && cfg[2] > 0) ? cfg[2] : 0;
   a.sb = 0;

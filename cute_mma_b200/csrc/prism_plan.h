@@ -1,0 +1,73 @@
+// Launch plans that follow from sizes alone: tile widths of the forward and dB.  Host code without CUDA, so that the rules can
+// be called where there is no GPU.
+#pragma once
+
+namespace prism {
+
+// Widest n-tile of a group: the largest multiple of 32 up to 256 that divides group_size, or 16; 0 where there is none.  A
+// narrow tile reloads A and repeats the rotation and the gate for every tile of the group.
+// Measured against the powers of two used before, 2000 x 3000 -> 6144 with groups of 192 (64 -> 192 wide): forward 218 ->
+// 92 us, dB 323 -> 134 us; 1000 x 1000 -> 1440 with groups of 96 (32 -> 96): 31 -> 17 and 40 -> 16 us.  Widths that are
+// multiples of 16 only are left at 16.
+inline int default_bn(int gs) {
+  for (int c = 256; c >= 32; c -= 32)
+    if (gs % c == 0) return c;
+  return gs % 16 == 0 ? 16 : 0;
+}
+
+// Widest power of two up to 256 that divides group_size (a multiple of 16).
+inline int pow2_bn(int gs) {
+  int bn = 256;
+  while (gs % bn != 0) bn /= 2;
+  return bn;
+}
+
+inline long long fwd_tiles(int M, int N, int bn) { return (long long)((M + 255) / 256) * (N / bn); }
+
+// Estimated time (us) of the general forward with tiles of bn columns: waves of CTA pairs x (64-wide chunks of K x the time of
+// one + epilogue).  A chunk takes 0.41 us at 64 columns, 0.44 at 128, 0.48 at 192 and 0.57 at 256; the epilogue 0.007 us a
+// column by TMA stores (multiples of 64), 0.0145 by plain ones, and 0.010 and 0.034 with a bias, which only the former
+// stages in shared memory (waves of 74 tiles of 256 rows, 2 to 32 chunks).
+inline double fwd_tile_us(int M, int N, int K, int bn, bool bias, int pairs) {
+  const double w = bn / 256.0;
+  const double epilogue = bn % 64 == 0 ? (bias ? 0.010 : 0.007) * bn : (bias ? 0.034 : 0.0145) * bn;
+  return (double)((fwd_tiles(M, N, bn) + pairs - 1) / pairs) * ((K + 63) / 64 * (0.40 + 0.17 * w * w) + epilogue);
+}
+
+// n-tile of the general forward.  A narrow tile repeats its group's rotation and gate, but on a CTA pair that would be idle,
+// and its epilogue is shorter.
+// Groups whose widest tile is a power of two: that tile, halved (down to 64) as long as the narrower tiles still run in one
+// wave.  Measured, 256 against 64 wide: 1024 x 256 -> 1024 8.9 / 7.1 us, 1024 x 768 -> 768 12.8 / 10.7; 200 x 4096 -> 1024
+// 32.6 / 30.4; 32 wide is no faster (8.8, 15.7, 30.3), and two waves lose (128 x 4096 -> 14336: 36.7 / 104.9).
+// Other groups (96, 160, 192, 224, ...): of the widest tile, the widest power of two and the multiples of 64 between, the
+// one with the least estimated time, the wider of two within 3 %.  The widest alone lost to the powers of two in short calls,
+// the more so with a bias: 207 x 496 -> 448 with groups of 224, 224 / 32 wide 11.8 / 8.5 us, with a bias 15.2 / 9.0; 300 x 1024 -> 768 with
+// groups of 192, 96 / 64 wide 13.7 / 12.2 us with a bias.  Over 600 drawn shapes with and without a bias the rule takes 0.4 %
+// longer than the best width in the mean; the widest tile halved to fit took 5.8 %, powers of two 26 %.
+inline int fwd_default_bn(int M, int N, int K, int gs, bool bias, int sms) {
+  const int pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const int widest = default_bn(gs), pow2 = pow2_bn(gs);
+  int best = widest;
+  if (widest == pow2) {
+    while (best >= 128 && fwd_tiles(M, N, best / 2) <= pairs) best /= 2;
+    return best;
+  }
+  double best_us = fwd_tile_us(M, N, K, widest, bias, pairs);
+  for (int c = widest - 32; c >= 16; c -= 16) {
+    if (gs % c != 0 || (c % 64 != 0 && c != pow2)) continue;
+    const double us = fwd_tile_us(M, N, K, c, bias, pairs);
+    if (us < 0.97 * best_us) { best = c; best_us = us; }
+  }
+  return best;
+}
+
+// Whether the general forward widens rotations of 8 itself or gets a widened copy of R from a launch before it (about 2 us,
+// and its host time): itself where a CTA pair has few chunks of 64 features to go through.  Measured, copy against
+// itself: 4 chunks 10.3 -> 9.1 us, 12 chunks 12.7 -> 11.9, 16 chunks 14.5 -> 13.9; 132 chunks (plain mode) 80 -> 78-81;
+// 448 chunks 269 -> 318, 448 of a deeper layer 228 -> 303.
+inline bool fwd_widens(int M, int N, int K, int bn, int sms) {
+  const long long tiles = fwd_tiles(M, N, bn), pairs = sms / 2 > 0 ? sms / 2 : 1;
+  return (tiles + pairs - 1) / pairs * ((K + 63) / 64) <= 32;
+}
+
+}  // namespace prism

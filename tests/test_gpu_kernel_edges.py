@@ -327,7 +327,7 @@ def test_rotations_of_8_are_widened_in_the_forward(M, K, path, act):
 
 @pytest.mark.parametrize("M,N,gs", [(1, 256, 256), (257, 1024, 256), (256, 18944, 256), (300, 768, 192), (64, 512, 512)])
 def test_tile_width_of_short_forwards(M, N, gs):
-    """Narrow tiles while they fit one wave (74 tiles of 256: none; groups of 192: 96 wide) give the bits of wide ones."""
+    """Narrow tiles while they fit one wave (74 tiles of 256: none; groups of 192: 64 wide) give the bits of wide ones."""
     K, rs, dt = 200, 8, torch.float16
     A, B, R, _ = _inputs(M, K, N, gs, rs, dt, 21)
     bias = torch.randn(N, device=DEV).to(dt)
