@@ -3,7 +3,6 @@
 #include "../../include/prism_b200.h"
 #include "prism_host.cuh"
 #include "prism_kernels.cuh"
-#include "prism_plan.h"
 
 namespace prism {
 
@@ -249,12 +248,11 @@ extern "C" size_t prism_workspace_bytes(int kind, int M, int N, int K, int gs, i
     return bytes;
   }
   if (kind == PRISM_KIND_BWD_DB) {
-    const int bn = (cfg && cfg[0] > 0) ? cfg[0] : default_bn(gs);
-    if (bn <= 0) return bytes;
+    if (default_bn(gs) == 0) return bytes;
     DbPlan pl;
-    db_plan(M, N, K, bn, num_sms(), cfg, &pl);
+    db_plan(M, N, K, gs, num_sms(), cfg, &pl);
     if (pl.splits > 1) bytes += align256((size_t)pl.splits * N * K * 4);
-    else if (pl.tail_rows > 0) bytes += align256((size_t)pl.tail_splits * pl.tail_rows * bn * K * 4);
+    else if (pl.tail_rows > 0) bytes += align256((size_t)pl.tail_splits * pl.tail_rows * pl.bn * K * 4);
     return bytes;
   }
   if (kind == PRISM_KIND_BWD_DADR || kind == PRISM_KIND_BWD_DADR_IB) {
@@ -399,11 +397,10 @@ extern "C" int prism_bwd_db_mask(const void* dC, const void* A, const void* R, c
   a.lddc = lddc; a.lda = lda; a.lddb = lddb;
   a.R = R; a.ldr = ldr; a.widen = rs == 8 ? 1 : 0;
   uint8_t* wp = reinterpret_cast<uint8_t*>(workspace) + PRISM_WORKSPACE_HEADER_BYTES;
-  a.BN = (cfg && cfg[0] > 0) ? cfg[0] : default_bn(gs);
-  if (a.BN % 16 != 0 || a.BN > 256 || gs % a.BN != 0)
-    return fail(PRISM_ERR_BAD_ARG, "%s: tile BN=%d must be a multiple of 16, <= 256 and divide group_size=%d", fn, a.BN, gs);
   a.num_sms = num_sms();
-  db_plan(M, N, K, a.BN, a.num_sms, cfg, &a.plan);
+  db_plan(M, N, K, gs, a.num_sms, cfg, &a.plan);
+  if (a.plan.bn % 16 != 0 || a.plan.bn > 256 || gs % a.plan.bn != 0)
+    return fail(PRISM_ERR_BAD_ARG, "%s: tile BN=%d must be a multiple of 16, <= 256 and divide group_size=%d", fn, a.plan.bn, gs);
   a.partial = (a.plan.splits > 1 || a.plan.tail_rows > 0) ? reinterpret_cast<float*>(wp) : nullptr;
   a.err = reinterpret_cast<int*>(workspace);
   a.stream = s;

@@ -369,57 +369,12 @@ __global__ void db_reduce_kernel(const float* __restrict__ partial, void* __rest
     *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dB_out) + (long long)n * lddb + k) = Elem<DT>::pack(acc.x, acc.y);
 }
 
-// Token-range splits of every tile: the count with the least estimated time, in units of one token block of a CTA pair
-// (about 1.1 us at BN = 256): waves of pairs x (blocks per pair + 3 for a pair's start and epilogue), and, when split, the
-// second launch with the fp32 partial sums written and read once (8 bytes each, about 6 TB/s).  Splitting pays when the
-// tiles leave most SM pairs idle; a count that only turns one wave into three shorter ones does not (4096 tokens, 1024 ->
-// 4096: 64 tiles on 74 pairs; three splits and their sum 69.5 us, none 41.2).
-static int db_default_splits(int M, int N, int K, int BN, int num_sms) {
-  const long long tiles = (long long)((K + 255) / 256) * (N / BN);
-  const int tokblocks = (M + 127) / 128;
-  const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
-  int best = 1;
-  double best_cost = 0;
-  for (int s = 1; s <= 16 && s <= tokblocks; ++s) {
-    const long long waves = (tiles * s + pairs - 1) / pairs;
-    double cost = (double)waves * ((tokblocks + s - 1) / s + 3);
-    if (s > 1) cost += 4.0 + (double)s * N * K * 8.0 / 6.6e6;
-    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
-  }
-  return best;
-}
-
-// Launch plan.  cfg = {BN, splits} or null: splits > 0 splits the token range of every tile, splits < 0
-// never splits.  Default: tiles that fill the GPU at least once are not split; when their count
-// leaves a last wave that is mostly empty, the last n-tile rows go to a second launch whose token
-// range is split so that it fills the GPU too (its partial sums cover those rows only).
-void db_plan(int M, int N, int K, int BN, int num_sms, const int* cfg, DbPlan* pl) {
-  pl->splits = 1; pl->tail_rows = 0; pl->tail_splits = 1;
-  const int user = cfg ? cfg[1] : 0;
-  if (user > 0) { pl->splits = user; return; }
-  if (user < 0 || BN <= 0) return;
-  pl->splits = db_default_splits(M, N, K, BN, num_sms);
-  if (pl->splits != 1) return;
-  const int x_pairs = (K + 255) / 256, rows = N / BN, slots = num_sms / 2 > 0 ? num_sms / 2 : 1;
-  const int tiles = x_pairs * rows, tokblocks = (M + 127) / 128;
-  if (tiles <= slots) return;
-  const int tail = tiles % slots;
-  if (tail == 0 || 2 * tail > slots) return;          // the last wave is full enough
-  const int yb = (tail + x_pairs - 1) / x_pairs;       // n-tile rows that hold the tail
-  int sb = slots / (yb * x_pairs);
-  if (sb > 16) sb = 16;
-  if (sb > tokblocks) sb = tokblocks;
-  if (sb < 2 || yb >= rows) return;
-  pl->tail_rows = yb;
-  pl->tail_splits = sb;
-}
-
 int launch_bwd_db(const DbArgs& a) {
   DbParams p;
-  p.M = a.M; p.N = a.N; p.K = a.K; p.gs = a.gs; p.E = a.E; p.BN = a.BN;
-  p.ntiles_per_group = a.gs / a.BN;
+  p.M = a.M; p.N = a.N; p.K = a.K; p.gs = a.gs; p.E = a.E; p.BN = a.plan.bn;
+  p.ntiles_per_group = a.gs / a.plan.bn;
   p.n_tokblocks = (a.M + 127) / 128;
-  p.dc_tiles = (a.BN / 2 + 63) / 64;   // per CTA: half of the tile's dC columns
+  p.dc_tiles = (a.plan.bn / 2 + 63) / 64;   // per CTA: half of the tile's dC columns
   p.r_tile_bytes = ((a.E * 128) + 1023) / 1024 * 1024;
   p.scale = a.scale; p.out_f32 = a.out_f32; p.ib = a.ib;
   p.R8 = a.widen ? reinterpret_cast<const uint16_t*>(a.R) : nullptr; p.ldr = a.ldr;
@@ -435,7 +390,7 @@ int launch_bwd_db(const DbArgs& a) {
   int ns = db::kMaxStages;
   while (ns > 2 && ns * p.stage_bytes > budget) --ns;
   if (ns * p.stage_bytes > budget)
-    return fail(PRISM_ERR_UNSUPPORTED, "bwd_db tile does not fit shared memory (BN=%d E=%d)", a.BN, a.E);
+    return fail(PRISM_ERR_UNSUPPORTED, "bwd_db tile does not fit shared memory (BN=%d E=%d)", a.plan.bn, a.E);
   p.ns = ns;
   const int smem_bytes = 2 * p.r_tile_bytes + ns * p.stage_bytes + (int)sizeof(DbBarriers) + 1024;
 
@@ -445,7 +400,7 @@ int launch_bwd_db(const DbArgs& a) {
   if ((rc = make_tmap_2d(&tmR, a.dtype, a.R, (uint64_t)(a.N / a.gs) * (a.widen ? 8 : a.E), a.K, a.ldr, a.widen ? 8 : a.E, 64, true))) return rc;
   if ((rc = make_tmap_2d(&tmdC, a.dtype, a.dC, a.M, a.N, a.lddc, 128, 64, true))) return rc;
 
-  p.box_rows = a.BN % 64 == 0 ? 64 : a.BN % 32 == 0 ? 32 : 16;
+  p.box_rows = a.plan.bn % 64 == 0 ? 64 : a.plan.bn % 32 == 0 ? 32 : 16;
   if (a.out_f32) tmdB = tmdC;   // not used
   else if ((rc = make_tmap_2d(&tmdB, a.dtype, a.dB, a.N, a.K, a.lddb, p.box_rows, 64, true))) return rc;
 
@@ -464,12 +419,12 @@ int launch_bwd_db(const DbArgs& a) {
 #undef PRISM_PICK_W
 #undef PRISM_PICK_G
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_db"))) return rc;
-  const int rows = a.N / a.BN;
+  const int rows = a.N / a.plan.bn;
   // one launch over the n-tile rows [nt0, nt0 + nrows) with the token range of every tile split `splits` ways
   auto launch = [&](int nt0, int nrows, int splits) -> int {
     DbParams q = p;
     q.nt0 = nt0;
-    q.part_rows = nrows * a.BN;
+    q.part_rows = nrows * a.plan.bn;
     q.blocks_per_split = (p.n_tokblocks + splits - 1) / splits;
     q.splits = (p.n_tokblocks + q.blocks_per_split - 1) / q.blocks_per_split;   // drop splits that would own no token block
     dim3 grid(2 * ((a.K + 255) / 256), nrows, q.splits);   // x: CTA pairs of 2 x 128 features
@@ -480,7 +435,7 @@ int launch_bwd_db(const DbArgs& a) {
       const long long pairs = (long long)q.part_rows * a.K / 2;
       const int threads = 256;
       const long long blocks = (pairs + threads - 1) / threads;
-      void* out = reinterpret_cast<uint8_t*>(a.dB) + (long long)nt0 * a.BN * a.lddb * (a.out_f32 ? 4 : 2);
+      void* out = reinterpret_cast<uint8_t*>(a.dB) + (long long)nt0 * a.plan.bn * a.lddb * (a.out_f32 ? 4 : 2);
 #define PRISM_DB_REDUCE(DT_, F32_) \
   db_reduce_kernel<DT_, F32_><<<(unsigned)blocks, threads, 0, a.stream>>>(a.partial, out, q.part_rows, a.K, a.lddb, q.splits)
       if (a.dtype == DT_BF16) { if (a.out_f32) PRISM_DB_REDUCE(DT_BF16, true); else PRISM_DB_REDUCE(DT_BF16, false); }

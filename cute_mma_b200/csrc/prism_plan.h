@@ -70,4 +70,80 @@ inline bool fwd_widens(int M, int N, int K, int bn, int sms) {
   return (tiles + pairs - 1) / pairs * ((K + 63) / 64) <= 32;
 }
 
+// Launch plan of the dB kernel: tile width, and how the token range of the tiles is split.
+struct DbPlan {
+  int bn;           // outputs per tile
+  int splits;       // token-range splits of every tile (1: none)
+  int tail_rows;    // n-tile rows of a mostly empty last wave that go to a second launch (0: none) ...
+  int tail_splits;  // ... with their token range split this often
+};
+
+inline int db_tokblocks(int M) { return M > 128 ? (M - 1) / 128 + 1 : 1; }
+
+// Estimated time (us) of one launch over `rows` n-tile rows: waves of CTA pairs x (token blocks x the time of one + a pair's
+// start and epilogue).  A block of 128 tokens takes 0.97 us up to 128 outputs a tile, 1.15 at 192, 1.30 at 256; start and
+// epilogue 4.4 us at 16 outputs, 5.8 at 256 (74 to 444 tiles, 1 to 64 blocks; rotations of 8 to 32 and both 16-bit types
+// alike, rotations of 64 up to 11 % longer).  A split launch has its sum after it, with the fp32 partial sums written and read
+// once: 10 TB/s while they stay in L2, 6.4 from memory.
+inline double db_launch_us(int M, int K, int rows, int bn, int splits, int pairs) {
+  const int tokblocks = db_tokblocks(M);
+  const int per = (tokblocks + splits - 1) / splits;
+  splits = (tokblocks + per - 1) / per;   // splits that would own no token block are dropped
+  const long long tiles = (long long)((K + 255) / 256) * rows * splits;
+  const double block = 0.97 + (bn > 128 ? 0.0026 * (bn - 128) : 0.0);
+  double us = (double)((tiles + pairs - 1) / pairs) * (per * block + 4.3 + 0.006 * bn) + 1.0;
+  if (splits > 1) {
+    const double bytes = 8.0 * splits * rows * bn * K;
+    us += 2.0 + 0.1 * splits + bytes / (bytes < 64e6 ? 10e6 : 6.4e6);
+  }
+  return us;
+}
+
+// The last wave's n-tile rows and their splits, where that wave is at most half full and another launch can fill it.
+inline bool db_tail(int M, int N, int K, int bn, int pairs, int* tail_rows, int* tail_splits) {
+  const int x_pairs = (K + 255) / 256, rows = N / bn, tokblocks = db_tokblocks(M);
+  const int tiles = x_pairs * rows, tail = tiles % pairs;
+  if (tiles <= pairs || tail == 0 || 2 * tail > pairs) return false;
+  const int yb = (tail + x_pairs - 1) / x_pairs;
+  int sb = pairs / (yb * x_pairs);
+  if (sb > 16) sb = 16;
+  if (sb > tokblocks) sb = tokblocks;
+  if (sb < 2 || yb >= rows) return false;
+  *tail_rows = yb;
+  *tail_splits = sb;
+  return true;
+}
+
+// cfg = {bn, splits} or null, 0 = default; splits > 0 splits the token range of every tile, splits < 0 never splits.
+// Default: the plan with the least estimated time of no splits, 2 to 16 splits of every tile, and splits of the rows of a mostly
+// empty last wave only, each with the widest tile and with the widest power of two that divides the group.
+// Over 500 timed shapes (16 to 512 outputs a group, both widths, up to 12 plans each) the rule is 0.2 % above the best plan in
+// the mean.  Two rules before it: splits until the tiles fill the GPU twice, powers of two (59 % above); the widest tile and one
+// time for a block of any width, tails not compared with splits of everything (3 %, up to 29 %: 10031 x 1728 -> 2816, groups of
+// 64, 473 us split against 413 with a split tail).
+inline void db_plan(int M, int N, int K, int gs, int sms, const int* cfg, DbPlan* pl) {
+  const int pairs = sms / 2 > 0 ? sms / 2 : 1, tokblocks = db_tokblocks(M);
+  const int user_bn = cfg ? cfg[0] : 0, user = cfg ? cfg[1] : 0;
+  const int widths[2] = {user_bn > 0 ? user_bn : default_bn(gs), user_bn > 0 ? user_bn : pow2_bn(gs)};
+  pl->bn = widths[0]; pl->splits = 1; pl->tail_rows = 0; pl->tail_splits = 1;
+  if (user > 0) pl->splits = user;
+  double best = 0;
+  for (int i = 0; i < (widths[1] != widths[0] ? 2 : 1); ++i) {
+    const int bn = widths[i], rows = N / bn;
+    auto consider = [&](double us, int splits, int tail_rows, int tail_splits) {
+      if (best > 0 && us >= best) return;
+      best = us;
+      pl->bn = bn; pl->splits = splits; pl->tail_rows = tail_rows; pl->tail_splits = tail_splits;
+    };
+    if (user != 0) {
+      consider(db_launch_us(M, K, rows, bn, user > 0 ? user : 1, pairs), user > 0 ? user : 1, 0, 1);
+      continue;
+    }
+    for (int s = 1; s <= 16 && s <= tokblocks; ++s) consider(db_launch_us(M, K, rows, bn, s, pairs), s, 0, 1);
+    int yb, sb;
+    if (db_tail(M, N, K, bn, pairs, &yb, &sb))
+      consider(db_launch_us(M, K, rows - yb, bn, 1, pairs) + db_launch_us(M, K, yb, bn, sb, pairs), 1, yb, sb);
+  }
+}
+
 }  // namespace prism

@@ -3,3 +3,8 @@
 
 extern "C" int plan_fwd_bn(int M, int N, int K, int gs, int bias, int sms) { return prism::fwd_default_bn(M, N, K, gs, bias != 0, sms); }
 extern "C" double plan_fwd_us(int M, int N, int K, int bn, int bias, int sms) { return prism::fwd_tile_us(M, N, K, bn, bias != 0, sms / 2); }
+extern "C" void plan_db(int M, int N, int K, int gs, int sms, const int* cfg, int* out) {
+  prism::DbPlan p;
+  prism::db_plan(M, N, K, gs, sms, cfg, &p);
+  out[0] = p.bn; out[1] = p.splits; out[2] = p.tail_rows; out[3] = p.tail_splits;
+}

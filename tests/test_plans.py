@@ -40,3 +40,40 @@ def test_forward_tile_widths_are_ones_the_kernel_takes(plan, gs, bias):
     (256, 512, 18944, 256, 0, 256), (300, 512, 4608, 512, 1, 128), (64, 512, 512, 32, 1, 32), (64, 512, 528, 48, 1, 16)])
 def test_forward_tile_width(plan, M, K, N, gs, bias, bn):
     assert plan.plan_fwd_bn(M, N, K, gs, bias, SMS) == bn
+
+
+def _db(plan, M, N, K, gs, cfg=None):
+    out = (ctypes.c_int * 4)()
+    plan.plan_db(M, N, K, gs, SMS, None if cfg is None else (ctypes.c_int * 8)(*cfg), out)
+    return tuple(out)
+
+
+@pytest.mark.parametrize("gs", range(16, 1040, 16))
+def test_plans_of_db_are_ones_the_kernel_takes(plan, gs):
+    for M in (0, 1, 128, 129, 4096, 16384):
+        for n in (1, 3, 40, 200):
+            for K in (8, 264, 4096):
+                bn, splits, tail_rows, tail_splits = _db(plan, M, n * gs, K, gs)
+                assert bn % 16 == 0 and 16 <= bn <= 256 and gs % bn == 0
+                assert 1 <= splits <= 16 and splits <= max(1, (M + 127) // 128)
+                assert tail_rows == 0 or (splits == 1 and 0 < tail_rows < n * gs // bn and 2 <= tail_splits <= 16)
+
+
+@pytest.mark.parametrize("M,K,N,gs,want", [
+    (128, 256, 256, 256, (256, 1, 0, 1)),         # one token block
+    (4096, 1024, 4096, 256, (256, 1, 0, 1)),      # 64 tiles, one wave: three splits would make three waves
+    (2200, 256, 256, 128, (128, 9, 0, 1)),        # two tiles, 18 token blocks: as often as it pays
+    (8192, 1024, 5120, 256, (256, 1, 2, 9)),      # 80 tiles: the last wave's rows are split, not everything
+    (16384, 1024, 5120, 256, (256, 1, 2, 9)),
+    (10031, 1728, 2816, 64, (64, 1, 2, 5)),       # narrow tiles: a block takes 0.97 us, not 1.3
+    (61, 464, 224, 224, (32, 1, 0, 1)),           # one block and few tiles: narrow ones
+    (2000, 3000, 6144, 192, (192, 1, 2, 3)),      # 384 tiles, the last of six waves 14
+    (16384, 4096, 14336, 256, (256, 1, 1, 4))])  # 896 tiles
+def test_plan_of_db(plan, M, K, N, gs, want):
+    assert _db(plan, M, N, K, gs) == want
+
+
+def test_plan_of_db_given_by_hand(plan):
+    assert _db(plan, 4096, 4096, 1024, 256, [128, 3, 0, 0, 0, 0, 0, 0]) == (128, 3, 0, 1)
+    assert _db(plan, 8192, 5120, 1024, 256, [0, -1, 0, 0, 0, 0, 0, 0]) == (256, 1, 0, 1)
+    assert _db(plan, 0, 4096, 1024, 256, [0, 4, 0, 0, 0, 0, 0, 0])[1] == 4
