@@ -436,10 +436,23 @@ def _dropout_mask(seeds, p, M, N, K, group_size):
 def _backward_both(dC, A, B, R, group_size, reconn_sz, gate, dc_scale=1.0, need_dB=True, internal_bias=None, seeds=None,
                    dropout_p=0.0, tile_cfg_dadr=None, tile_cfg_db=None, dR_dtype=None, dB_dtype=None):
     """(dA, dR, dB, d_internal_bias) by the dA+dR kernel and, in the gated modes where dB is wanted, the dB kernel; None for
-    what there is none of.  The dropout mask that the first leaves for the second is only an economy: where its memory
-    is needed for anything else of the two calls, it is given back and the dB kernel hashes for itself."""
+    what there is none of."""
     need_dB = need_dB and gate != 0
-    mask = _dropout_mask(seeds, dropout_p, A.shape[0], B.shape[0], A.shape[1], group_size) if need_dB else None
+    if seeds is not None:
+        out, dB = _backward_with_dropout(dC, A, B, R, (group_size, reconn_sz, gate, dc_scale), need_dB, internal_bias, seeds,
+                                         dropout_p, tile_cfg_dadr, tile_cfg_db, dR_dtype, dB_dtype)
+    else:
+        out = _backward_dadr(dC, A, B, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_dadr, dR_dtype, internal_bias)
+        dB = (_backward_db(dC, A, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_db, dB_dtype, internal_bias)
+              if need_dB else None)
+    return out[0], out[1], dB, out[2] if internal_bias is not None else None
+
+
+def _backward_with_dropout(dC, A, B, R, args, need_dB, internal_bias, seeds, p, tile_cfg_dadr, tile_cfg_db, dR_dtype, dB_dtype):
+    """The mask that the dA+dR kernel leaves for the dB kernel is only an economy: where its memory is needed for anything
+    else of the two calls, it is given back and the dB kernel hashes for itself."""
+    mask = _dropout_mask(seeds, p, A.shape[0], B.shape[0], A.shape[1], args[0]) if need_dB else None
+    kw = dict(internal_bias=internal_bias, dropout_seeds=seeds, dropout_p=p)
 
     def without_mask_if_short(call):
         nonlocal mask
@@ -451,15 +464,10 @@ def _backward_both(dC, A, B, R, group_size, reconn_sz, gate, dc_scale=1.0, need_
         mask = None   # out here, where the failed call's frames are gone and with them their references to it
         return call(None)
 
-    out = without_mask_if_short(lambda m: _backward_dadr(
-        dC, A, B, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_dadr, dR_dtype, internal_bias=internal_bias,
-        dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=m))
-    dB = None
-    if need_dB:
-        dB = without_mask_if_short(lambda m: _backward_db(
-            dC, A, R, group_size, reconn_sz, gate, dc_scale, tile_cfg_db, dB_dtype, internal_bias=internal_bias,
-            dropout_seeds=seeds, dropout_p=dropout_p, dropout_mask=m))
-    return out[0], out[1], dB, out[2] if internal_bias is not None else None
+    out = without_mask_if_short(lambda m: _backward_dadr(dC, A, B, R, *args, tile_cfg_dadr, dR_dtype, dropout_mask=m, **kw))
+    dB = (without_mask_if_short(lambda m: _backward_db(dC, A, R, *args, tile_cfg_db, dB_dtype, dropout_mask=m, **kw))
+          if need_dB else None)
+    return out, dB
 
 
 def _out_buffer(out, shape, dtype, device, name):

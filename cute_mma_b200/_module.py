@@ -210,6 +210,9 @@ _prism_forward_op.register_autograd(_backward, setup_context=_setup_context)
 # ---------------------------------------------------------------------------
 # the eager path: one autograd node for the whole layer
 # ---------------------------------------------------------------------------
+_PLAIN_TYPES = (torch.Tensor, nn.Parameter)
+
+
 def _plain_eager(*tensors) -> bool:
     """Whether this call is ordinary eager work on CUDA tensors.  Tracing, compilation, dispatch and function modes, torch.func
     transforms, forward-mode differentiation and tensor subclasses have to see the custom ops, which describe themselves
@@ -224,7 +227,7 @@ def _plain_eager(*tensors) -> bool:
         return False
     for t in tensors:
         # (a view with the negative bit, as of a conjugate's imaginary part, is in memory what its values are not)
-        if t is not None and (type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda or t.is_neg()):
+        if t is not None and (type(t) not in _PLAIN_TYPES or not t.is_cuda or t.is_neg()):
             return False
     return True
 

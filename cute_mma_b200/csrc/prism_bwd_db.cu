@@ -19,8 +19,8 @@
 //   warps 4-19  gate warps, 16 token rows x 64 features each: S from TMEM, A by ldmatrix, H = A*silu(S)
 //               on registers, stmatrix of H over the A tile in place
 //               Dense product D += H^T . dC as 8 x tcgen05.mma M256 N=BN K=16 per token block.
-//   warps 20-23 epilogue: D -> dB (transposed by stmatrix into the stages' memory, TMA stores), fp32 dB, or fp32
-//               partials when the token range is split;
+//   warps 20-23 epilogue: D -> dB (TMA_OUT: transposed by stmatrix into the stages' memory, TMA stores; else 2-byte stores),
+//               fp32 dB, or fp32 partials when the token range is split;
 //               a second kernel then adds the partials in a fixed order (deterministic).
 // Both products run on tcgen05: mma.sync would share the tensor cores with tcgen05.mma and starve
 // behind it.
@@ -41,32 +41,40 @@ constexpr int kSCol0 = 256;        // accumulator: TMEM columns [0, 256); S: [25
 }  // namespace db
 
 struct DbParams {
-  int M, N, K, gs, E, BN;
+  int K, BN;
   int ntiles_per_group;
   int blocks_per_split, n_tokblocks;
   int dc_tiles;       // ceil(BN / 128): 64-column dC tiles per CTA
-  int r_tile_bytes;   // bytes reserved per R tile (multiple of 1024)
   int ns;             // stages: two A tiles + this CTA's dC tiles
   int stage_bytes;
   int splits;
   int out_f32;        // 1: dB is fp32
   int box_rows;       // rows of dB per TMA store of the epilogue (divides BN)
+  int nt0;            // first n-tile of this launch (blockIdx.y counts from it)
+  int part_rows;      // output rows covered by the partial buffer, starting at row nt0 * BN
   float scale;
-  const uint16_t* R8; // reconn_sz 8: R [G*8, K] itself, or null: the R tiles come through tmR
+  uint32_t drop_thr;   // see drop_threshold
+  float drop_inv_keep;
+  const uint16_t* R8; // reconn_sz 8: R [G*8, K] itself, else null: the R tiles come through DbMaps::R
   long long ldr;
   const void* ib;     // internal bias [G, K] or null
   const long long* drop_seeds;   // per-group dropout seeds (DROP kernels)
-  uint32_t drop_thr;   // see drop_threshold
-  float drop_inv_keep;
   const uint32_t* drop_mask;   // the masks as the dA+dR kernel left them (prism_dropout_mask_bytes), or null: hash again
-  int n_k64;
-  void* dB;
+  void* out;          // dB, or the partial sums [splits][part_rows][K] fp32 when splits > 1
   long long lddb;
-  float* partial;     // [splits][part_rows][K] when splits > 1
-  int nt0;            // first n-tile of this launch (blockIdx.y counts from it)
-  int part_rows;      // output rows covered by the partial buffer, starting at row nt0 * BN
   int* err;
 };
+
+// The kernel's tensor maps.  With three of them and DbParams the parameters are 512 bytes; beyond that the plain instances took
+// up to 0.035 us longer for every token block of a narrow tile, whatever the parameters held (two unused ones more: 8192 x
+// 256, groups of 32, sigmoid, 62.3 -> 65.3 us; 1497 x 2992 -> 7488, groups of 48, 1121 -> 1148), also in another order or copied to
+// registers first.
+template <bool TMA_OUT>
+struct DbMaps { CUtensorMap A, R, dC; };
+template <>
+struct DbMaps<true> { CUtensorMap A, R, dC, dB; };
+static_assert(sizeof(DbMaps<false>) + sizeof(DbParams) <= 512, "");
+
 
 struct DbBarriers {
   uint64_t r_full;                     // local: this CTA's R tiles landed (once)
@@ -80,18 +88,19 @@ struct DbBarriers {
 };
 
 // WIDEN: reconn_sz 8, R is widened here (E = 16); an instance of its own (see prism_fwd_small.cu)
-template <int DT, int GATE, int E, bool DROP, bool WIDEN>
+// TMA_OUT: unsplit 16-bit dB leaves by TMA stores (see db_tma_out)
+template <int DT, int GATE, int E, bool DROP, bool WIDEN, bool TMA_OUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(db::kThreads, 1)
-prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmR,
-                    const __grid_constant__ CUtensorMap tmdC, const __grid_constant__ CUtensorMap tmdB, const DbParams p) {
+prism_bwd_db_kernel(const __grid_constant__ DbMaps<TMA_OUT> tm, const DbParams p) {
   using namespace db;
   constexpr int KS = E / 16;    // K16 steps per rotation block
+  constexpr int kRTile = (E * 128 + 1023) / 1024 * 1024;
   constexpr int NBLK = 128 / E; // rotation blocks of this CTA's 128 features
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   uint8_t* smemR = smem;                           // two R tiles [E x 64]
-  uint8_t* smemSt = smemR + 2 * p.r_tile_bytes;    // stages: [A tile f0.. | A tile f0+64.. | dC tiles]
+  uint8_t* smemSt = smemR + 2 * kRTile;    // stages: [A tile f0.. | A tile f0+64.. | dC tiles]
   DbBarriers* bars = reinterpret_cast<DbBarriers*>(smemSt + p.ns * p.stage_bytes);
 
   const int warp = threadIdx.x >> 5;
@@ -125,7 +134,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if ((c & 1) == (i >> 3) && col < p.K)
       v = __ldg(reinterpret_cast<const uint4*>(p.R8 + (long long)(g * 8 + (i & 7)) * p.ldr + col));
-    *reinterpret_cast<uint4*>(smemR + t * p.r_tile_bytes + sw128_offset(i, c)) = v;
+    *reinterpret_cast<uint4*>(smemR + t * kRTile + sw128_offset(i, c)) = v;
     fence_proxy_async_smem();   // read by the rotation's MMAs, after the cluster barrier below
   }
   if (warp == kWarpMma) {
@@ -133,9 +142,9 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tmem_relinquish_pair();
   }
   if (warp == kWarpTma && lane == 0) {
-    prefetch_tmap(&tmA);
-    prefetch_tmap(&tmR);
-    prefetch_tmap(&tmdC);
+    prefetch_tmap(&tm.A);
+    prefetch_tmap(&tm.R);
+    prefetch_tmap(&tm.dC);
   }
   // the peer's barriers must be initialised before anything arrives on them remotely
   tc_fence_before_sync();
@@ -151,8 +160,8 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       bool ok = true;
       if (!WIDEN) {
         mbar_arrive_expect_tx(&bars->r_full, 2 * E * 128);
-        tma_load_2d(smemR, &tmR, &bars->r_full, f0, g * E);
-        tma_load_2d(smemR + p.r_tile_bytes, &tmR, &bars->r_full, f0 + 64, g * E);
+        tma_load_2d(smemR, &tm.R, &bars->r_full, f0, g * E);
+        tma_load_2d(smemR + kRTile, &tm.R, &bars->r_full, f0 + 64, g * E);
         // the rotation issuer (leader) reads the peer's R tiles too: it learns of them through the peer's
         // first A tiles, which are issued after this wait
         if (!mbar_wait(&bars->r_full, 0)) ok = false;
@@ -165,12 +174,12 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         // completion is counted on the leader's barriers: its MMAs read both CTAs' tiles
         const uint32_t afull = mapa_shared(smem_u32(&bars->a_full[rs.idx]), 0);
         mbar_arrive_expect_tx_cluster(afull, 2 * kTile);
-        tma_load_2d_pair(dst, &tmA, afull, f0, tok0);
-        tma_load_2d_pair(dst + kTile, &tmA, afull, f0 + 64, tok0);
+        tma_load_2d_pair(dst, &tm.A, afull, f0, tok0);
+        tma_load_2d_pair(dst + kTile, &tm.A, afull, f0 + 64, tok0);
         const uint32_t hdfull = mapa_shared(smem_u32(&bars->hd_full[rs.idx]), 0);
         mbar_arrive_expect_tx_cluster(hdfull, p.dc_tiles * kTile);
         for (int t = 0; t < p.dc_tiles; ++t)   // this CTA's half of the dC columns
-          tma_load_2d_pair(dst + (2 + t) * kTile, &tmdC, hdfull, n0 + (int)rank * (p.BN / 2) + 64 * t, tok0);
+          tma_load_2d_pair(dst + (2 + t) * kTile, &tm.dC, hdfull, n0 + (int)rank * (p.BN / 2) + 64 * t, tok0);
       }
       if (!ok) { atomicExch(p.err, PRISM_ERR_DEVICE_WAIT); }
     }
@@ -186,7 +195,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const uint64_t dr0 = desc_kmajor_sw128(smem_u32(smemR), 1024);
       const uint32_t k_hi = (uint32_t)(da0 >> 32);
       const uint32_t st_step = (uint32_t)p.stage_bytes >> 4;
-      const uint32_t r_step = (uint32_t)p.r_tile_bytes >> 4;
+      const uint32_t r_step = (uint32_t)kRTile >> 4;
       const uint32_t s0 = tmem_base + kSCol0;
       bool ok = true;
       Ring rr(p.ns);
@@ -258,7 +267,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       if (DROP) {   // before the wait: neither needs anything that is being loaded
         if (p.drop_mask != nullptr) {
           const long long m16 = (long long)(tb0 + j) * 8 + (int)(r0 >> 4);
-          mask = kvalid > 0 ? __ldg(p.drop_mask + (((long long)g * p.n_tokblocks * 8 + m16) * p.n_k64 + (kcol >> 6)) * 32 + lane) : 0u;
+          mask = kvalid > 0 ? __ldg(p.drop_mask + (((long long)g * p.n_tokblocks * 8 + m16) * ((p.K + 63) >> 6) + (kcol >> 6)) * 32 + lane) : 0u;
         } else {
           mask = drop_mask32(drop_h1, (uint64_t)((tb0 + j) * 128 + (int)r0 + (lane >> 2)) * p.K + kcol + 2 * (lane & 3),
                              8ull * p.K, p.drop_thr);
@@ -279,7 +288,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int q = warp & 3;
     const int f = f0 + q * 32 + lane;  // feature = accumulator row
     bool ok = mbar_wait(&bars->acc_full, 0);
-    if (p.splits == 1 && !p.out_f32) {
+    if constexpr (TMA_OUT) {
       // Every product has completed, so the stages' memory is free: box_rows rows of dB (outputs) by 2 x 64 features at a
       // time go there, each warp's 32 features transposed by stmatrix, and leave by TMA.  Two-byte stores from
       // the accumulator's rows, 64 bytes per instruction, took 1.3 us more per tile: 128 x 4096 -> 14336 118 -> 102 us,
@@ -311,7 +320,7 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         // the four epilogue warps, whether their wait ran out or not
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (ok && lane == 0 && q < 2 && f0 + q * 64 < p.K) {
-          tma_store_2d(&tmdB, smemSt + (2 * blk + q) * box_bytes, f0 + q * 64, n0 + c0);
+          tma_store_2d(&tm.dB, smemSt + (2 * blk + q) * box_bytes, f0 + q * 64, n0 + c0);
           tma_store_commit();
         }
       }
@@ -325,13 +334,20 @@ prism_bwd_db_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         tmem_ld_wait();
         if (f < p.K) {
           if (p.splits > 1) {
-            float* dst = p.partial + ((long long)split * p.part_rows + (n0 - p.nt0 * p.BN) + c0) * p.K + f;
+            float* dst = reinterpret_cast<float*>(p.out) + ((long long)split * p.part_rows + (n0 - p.nt0 * p.BN) + c0) * p.K + f;
 #pragma unroll
             for (int j = 0; j < 16; ++j) dst[(long long)j * p.K] = __uint_as_float(v[j]) * p.scale;
-          } else {
-            float* dst = reinterpret_cast<float*>(p.dB) + (long long)(n0 + c0) * p.lddb + f;
+          } else if (p.out_f32) {
+            float* dst = reinterpret_cast<float*>(p.out) + (long long)(n0 + c0) * p.lddb + f;
 #pragma unroll
             for (int j = 0; j < 16; ++j) dst[(long long)j * p.lddb] = __uint_as_float(v[j]) * p.scale;
+          } else {
+            uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (long long)(n0 + c0) * p.lddb + f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const uint32_t w = Elem<DT>::pack(__uint_as_float(v[j]) * p.scale, 0.f);
+              dst[(long long)j * p.lddb] = static_cast<uint16_t>(w & 0xFFFFu);
+            }
           }
         }
       }
@@ -369,56 +385,56 @@ __global__ void db_reduce_kernel(const float* __restrict__ partial, void* __rest
     *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dB_out) + (long long)n * lddb + k) = Elem<DT>::pack(acc.x, acc.y);
 }
 
+template <bool TMA_OUT>
+using DbKernel = void (*)(DbMaps<TMA_OUT>, DbParams);
+
+template <bool TMA_OUT>
+static DbKernel<TMA_OUT> db_kernel(const DbArgs& a, bool drop) {
+#define PRISM_PICK_W(DT_, E_, DROP_, W_)                                                                            \
+  (a.gate == GATE_SILU ? (DbKernel<TMA_OUT>)prism_bwd_db_kernel<DT_, GATE_SILU, E_, DROP_, W_, TMA_OUT>              \
+   : a.gate == GATE_SIGMOID ? (DbKernel<TMA_OUT>)prism_bwd_db_kernel<DT_, GATE_SIGMOID, E_, DROP_, W_, TMA_OUT>      \
+                            : (DbKernel<TMA_OUT>)prism_bwd_db_kernel<DT_, GATE_NONE, E_, false, W_, TMA_OUT>)
+#define PRISM_PICK(E_, DROP_, W_) return (a.dtype == DT_BF16) ? PRISM_PICK_W(DT_BF16, E_, DROP_, W_) : PRISM_PICK_W(DT_F16, E_, DROP_, W_)
+  if (a.widen) { if (drop) PRISM_PICK(16, true, true); else PRISM_PICK(16, false, true); }
+  if (drop) PRISM_PICK(16, true, false);
+  if (a.E == 16) PRISM_PICK(16, false, false);
+  if (a.E == 32) PRISM_PICK(32, false, false);
+  PRISM_PICK(64, false, false);
+#undef PRISM_PICK
+#undef PRISM_PICK_W
+}
+
 int launch_bwd_db(const DbArgs& a) {
   DbParams p;
-  p.M = a.M; p.N = a.N; p.K = a.K; p.gs = a.gs; p.E = a.E; p.BN = a.plan.bn;
+  p.K = a.K; p.BN = a.plan.bn;
   p.ntiles_per_group = a.gs / a.plan.bn;
   p.n_tokblocks = (a.M + 127) / 128;
   p.dc_tiles = (a.plan.bn / 2 + 63) / 64;   // per CTA: half of the tile's dC columns
-  p.r_tile_bytes = ((a.E * 128) + 1023) / 1024 * 1024;
+  const int r_tile_bytes = ((a.E * 128) + 1023) / 1024 * 1024;
   p.scale = a.scale; p.out_f32 = a.out_f32; p.ib = a.ib;
   p.R8 = a.widen ? reinterpret_cast<const uint16_t*>(a.R) : nullptr; p.ldr = a.ldr;
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
-  p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_mask = a.drop_mask; p.n_k64 = (a.K + 63) / 64; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
+  p.drop_seeds = a.drop_seeds; p.drop_thr = drop_threshold(a.drop_p); p.drop_mask = a.drop_mask; p.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "bwd_db: dropout needs reconn_sz 8 or 16");
-  p.dB = a.dB; p.lddb = a.lddb; p.partial = a.partial; p.err = a.err;
+  p.lddb = a.lddb; p.err = a.err;
   if ((a.plan.splits > 1 || a.plan.tail_rows > 0) && a.partial == nullptr)
     return fail(PRISM_ERR_WORKSPACE, "bwd_db: split accumulation needs a partial-sum workspace");
 
-  const int budget = 227 * 1024 - 1024 - (int)sizeof(DbBarriers) - 256 - 2 * p.r_tile_bytes;
+  const int budget = 227 * 1024 - 1024 - (int)sizeof(DbBarriers) - 256 - 2 * r_tile_bytes;
   p.stage_bytes = (2 + p.dc_tiles) * db::kTile;
   int ns = db::kMaxStages;
   while (ns > 2 && ns * p.stage_bytes > budget) --ns;
   if (ns * p.stage_bytes > budget)
     return fail(PRISM_ERR_UNSUPPORTED, "bwd_db tile does not fit shared memory (BN=%d E=%d)", a.plan.bn, a.E);
   p.ns = ns;
-  const int smem_bytes = 2 * p.r_tile_bytes + ns * p.stage_bytes + (int)sizeof(DbBarriers) + 1024;
+  const int smem_bytes = 2 * r_tile_bytes + ns * p.stage_bytes + (int)sizeof(DbBarriers) + 1024;
 
-  CUtensorMap tmA, tmR, tmdC, tmdB;
+  DbMaps<true> tm;
   int rc;
-  if ((rc = make_tmap_2d(&tmA, a.dtype, a.A, a.M, a.K, a.lda, 128, 64, true))) return rc;
-  if ((rc = make_tmap_2d(&tmR, a.dtype, a.R, (uint64_t)(a.N / a.gs) * (a.widen ? 8 : a.E), a.K, a.ldr, a.widen ? 8 : a.E, 64, true))) return rc;
-  if ((rc = make_tmap_2d(&tmdC, a.dtype, a.dC, a.M, a.N, a.lddc, 128, 64, true))) return rc;
-
+  if ((rc = make_tmap_2d(&tm.A, a.dtype, a.A, a.M, a.K, a.lda, 128, 64, true))) return rc;
+  if ((rc = make_tmap_2d(&tm.R, a.dtype, a.R, (uint64_t)(a.N / a.gs) * (a.widen ? 8 : a.E), a.K, a.ldr, a.widen ? 8 : a.E, 64, true))) return rc;
+  if ((rc = make_tmap_2d(&tm.dC, a.dtype, a.dC, a.M, a.N, a.lddc, 128, 64, true))) return rc;
   p.box_rows = a.plan.bn % 64 == 0 ? 64 : a.plan.bn % 32 == 0 ? 32 : 16;
-  if (a.out_f32) tmdB = tmdC;   // not used
-  else if ((rc = make_tmap_2d(&tmdB, a.dtype, a.dB, a.N, a.K, a.lddb, p.box_rows, 64, true))) return rc;
-
-  using KernT = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, DbParams);
-  KernT kern = nullptr;
-#define PRISM_PICK_W(DT_, E_, DROP_, W_)                                                                 \
-  (a.gate == GATE_SILU ? (KernT)prism_bwd_db_kernel<DT_, GATE_SILU, E_, DROP_, W_>                        \
-                       : a.gate == GATE_SIGMOID ? (KernT)prism_bwd_db_kernel<DT_, GATE_SIGMOID, E_, DROP_, W_> \
-                                                : (KernT)prism_bwd_db_kernel<DT_, GATE_NONE, E_, false, W_>)
-#define PRISM_PICK_G(E_, DROP_, W_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_W(DT_BF16, E_, DROP_, W_) : PRISM_PICK_W(DT_F16, E_, DROP_, W_)
-#define PRISM_PICK_16(DROP_) if (a.widen) { PRISM_PICK_G(16, DROP_, true); } else { PRISM_PICK_G(16, DROP_, false); }
-  if (drop) { PRISM_PICK_16(true) }
-  else if (a.E == 16) { PRISM_PICK_16(false) }
-  else if (a.E == 32) { PRISM_PICK_G(32, false, false); } else { PRISM_PICK_G(64, false, false); }
-#undef PRISM_PICK_16
-#undef PRISM_PICK_W
-#undef PRISM_PICK_G
-  if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_db"))) return rc;
   const int rows = a.N / a.plan.bn;
   // one launch over the n-tile rows [nt0, nt0 + nrows) with the token range of every tile split `splits` ways
   auto launch = [&](int nt0, int nrows, int splits) -> int {
@@ -427,9 +443,20 @@ int launch_bwd_db(const DbArgs& a) {
     q.part_rows = nrows * a.plan.bn;
     q.blocks_per_split = (p.n_tokblocks + splits - 1) / splits;
     q.splits = (p.n_tokblocks + q.blocks_per_split - 1) / q.blocks_per_split;   // drop splits that would own no token block
+    q.out = q.splits > 1 ? (void*)a.partial : a.dB;
     dim3 grid(2 * ((a.K + 255) / 256), nrows, q.splits);   // x: CTA pairs of 2 x 128 features
-    kern<<<grid, db::kThreads, smem_bytes, a.stream>>>(tmA, tmR, tmdC, tmdB, q);
     int rcl;
+    const bool bf16_silu = a.dtype == DT_BF16 && a.gate == GATE_SILU && !a.widen && !drop;
+    if (q.splits == 1 && !a.out_f32 && db_tma_out(a.plan.bn, q.blocks_per_split, bf16_silu)) {
+      if ((rcl = make_tmap_2d(&tm.dB, a.dtype, a.dB, a.N, a.K, a.lddb, p.box_rows, 64, true))) return rcl;
+      const DbKernel<true> kern = db_kernel<true>(a, drop);
+      if ((rcl = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_db"))) return rcl;
+      kern<<<grid, db::kThreads, smem_bytes, a.stream>>>(tm, q);
+    } else {
+      const DbKernel<false> kern = db_kernel<false>(a, drop);
+      if ((rcl = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_db"))) return rcl;
+      kern<<<grid, db::kThreads, smem_bytes, a.stream>>>(DbMaps<false>{tm.A, tm.R, tm.dC}, q);
+    }
     if ((rcl = check_launch("prism_bwd_db"))) return rcl;
     if (q.splits > 1) {
       const long long pairs = (long long)q.part_rows * a.K / 2;

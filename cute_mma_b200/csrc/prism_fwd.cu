@@ -127,8 +127,12 @@ __device__ __forceinline__ void epilogue_cols32(uint32_t tacc, uint8_t* stage, i
 }
 
 // EXTRA: 0 the plain gate warps; 1 internal bias (a null bias is allowed); 2 hash dropout (+ optional bias)
-// WIDEN: reconn_sz 8 in a short call, R is widened here (E = 16); an instance of its own, so that the others stay as they are
-template <int DT, int GATE, int E, int EXTRA, bool WIDEN>
+// WIDEN: reconn_sz 8 in a short call, R is widened here (E = 16).  An instance of its own, so that the others do not pay for the
+// choice at their start (0.2 to 0.4 us, see prism_fwd_small.cu).  Where the call is long the gate's loop decides, and the
+// instances that choose at run time have the faster one with dropout (4096 x 1024 -> 4096 at reconn_sz 16: 200 / 208 us) and in
+// the gated modes without internal bias (16384 x 4096 -> 14336: silu 1828 / 1848, sigmoid 1819 / 1830).
+enum FwdWiden { WIDEN_NO, WIDEN_YES, WIDEN_AT_RUN_TIME };
+template <int DT, int GATE, int E, int EXTRA, int WIDEN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(fwd::kThreads, 1)
 prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmR,
                  const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
@@ -136,6 +140,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   using namespace fwd;
   constexpr int KS = E / 16;   // K16 steps per rotation block
   constexpr int NB = 64 / E;   // rotation blocks per chunk
+  const bool widen = WIDEN == WIDEN_YES || (WIDEN == WIDEN_AT_RUN_TIME && p.R8 != nullptr);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
@@ -156,7 +161,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxStages; ++i) {
       // two producers in each CTA, one arrive.expect_tx each (and one arrive for a R tile written by warp 0)
-      mbar_init(&bars->loads_full[i], WIDEN ? 6 : 4);
+      mbar_init(&bars->loads_full[i], widen ? 6 : 4);
       mbar_init(&bars->done[i], 1);
     }
     for (int i = 0; i < kSlots; ++i) {
@@ -167,7 +172,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     mbar_init(&bars->acc_empty, 2 * kNumEpiWarps);
     fence_mbar_init();
   }
-  if (WIDEN) {
+  if (widen) {
     // the blocks off the widened diagonal stay zero for good: the producer only writes the others
     for (int i = threadIdx.x; i < p.ns * 64; i += kThreads)
       *reinterpret_cast<uint4*>(smemSt + (i >> 6) * p.stage_bytes + kATileBytes + (i & 63) * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -194,7 +199,7 @@ prism_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int my_tiles = (p.n_tiles - cid + n_clusters - 1) / n_clusters;
   const uint32_t total = (uint32_t)my_tiles * nk;   // chunks this CTA pair processes
 
-  if (WIDEN && warp == kWarpTma) {
+  if (widen && warp == kWarpTma) {
     // ------------------------------------------------------------------ producer for reconn_sz 8: A tile by TMA, R by hand
     // This CTA's eight rows of the widened R tile are R's eight rows of the group in every second piece of 8 features
     // (the leader the even ones, the peer the odd ones): one 16-byte piece per lane, fetched a chunk ahead.  For
@@ -541,10 +546,11 @@ int launch_fwd(const FwdArgs& a) {
                                                 : (KernT)prism_fwd_kernel<DT_, GATE_NONE, E_, 0, W_>)
 #define PRISM_PICK_G(E_, X_, W_) kern = (a.dtype == DT_BF16) ? PRISM_PICK_W(DT_BF16, E_, X_, W_) : PRISM_PICK_W(DT_F16, E_, X_, W_)
 #define PRISM_PICK(X_)                                                                                   \
-  if (a.widen) { PRISM_PICK_G(16, X_, true); } else if (a.E == 16) { PRISM_PICK_G(16, X_, false); }       \
-  else if (a.E == 32) { PRISM_PICK_G(32, X_, false); } else { PRISM_PICK_G(64, X_, false); }
+  if (a.widen) { PRISM_PICK_G(16, X_, WIDEN_YES); } else if (a.E == 16) { PRISM_PICK_G(16, X_, WIDEN_NO); } \
+  else if (a.E == 32) { PRISM_PICK_G(32, X_, WIDEN_NO); } else { PRISM_PICK_G(64, X_, WIDEN_NO); }
   const bool ib = a.ib != nullptr && a.gate != GATE_NONE;
-  if (drop) { if (a.widen) { PRISM_PICK_G(16, 2, true); } else { PRISM_PICK_G(16, 2, false); } }
+  if (drop) { PRISM_PICK_G(16, 2, WIDEN_AT_RUN_TIME); }
+  else if (a.E == 16 && !ib && a.gate != GATE_NONE && !fwd_widens(a.M, a.N, a.K, a.BN, a.num_sms)) { PRISM_PICK_G(16, 0, WIDEN_AT_RUN_TIME); }
   else if (ib) { PRISM_PICK(1) }
   else { PRISM_PICK(0) }
 #undef PRISM_PICK_W

@@ -131,8 +131,9 @@ int prism_bwd_dadr(const void* dC, const void* A, const void* B, const void* R, 
  * reference: dB_dtype, src/cute_prism/__init__.py:288-289,375).
  * cfg (2 ints, 0 = default): {BN, splits} -- splits > 1 divides the token range of every tile over
  * several CTA pairs whose fp32 partial sums (in the workspace) are added in a fixed order, so the
- * result is deterministic; splits < 0 never splits.  By default only the n-tile rows of a mostly
- * empty last wave are split (in a second launch). */
+ * result is deterministic; splits < 0 never splits.  By default the plan of
+ * least estimated time: no splits, splits of every tile, or of the n-tile rows of a mostly empty last wave only (in a
+ * second launch). */
 int prism_bwd_db(const void* dC, const void* A, const void* R, const void* internal_bias, void* dB,
                  int M, int N, int K, int group_size, int reconn_sz, int dtype, int gate,
                  int db_dtype, float dc_scale, long long lddc, long long lda, long long ldr, long long lddb,

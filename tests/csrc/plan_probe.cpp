@@ -8,3 +8,4 @@ extern "C" void plan_db(int M, int N, int K, int gs, int sms, const int* cfg, in
   prism::db_plan(M, N, K, gs, sms, cfg, &p);
   out[0] = p.bn; out[1] = p.splits; out[2] = p.tail_rows; out[3] = p.tail_splits;
 }
+extern "C" int plan_db_tma(int bn, int blocks, int bf16_silu) { return prism::db_tma_out(bn, blocks, bf16_silu != 0); }

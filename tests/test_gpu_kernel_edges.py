@@ -56,18 +56,28 @@ def test_widened_and_halved_rotation(K, rs):
         assert O.rel_err(got.float(), ref) < TOL
 
 
-@pytest.mark.parametrize("M,K,N,gs", [(128, 256, 256, 256),       # one token block: never split
-                                      (129, 272, 512, 256),       # two blocks, features past the first pair
-                                      (2200, 256, 256, 128),      # few tiles: split as often as it pays
-                                      (4096, 1024, 4096, 256)])   # 64 tiles: one wave, not split
+@pytest.mark.parametrize("M,K,N,gs,part_rows", [(128, 256, 256, 256, 0),           # one token block: never split
+                                                (129, 272, 512, 256, 0),           # two blocks, features past the first pair
+                                                (2200, 256, 256, 128, 9 * 256),    # few tiles: split as often as it pays
+                                                (4096, 1024, 4096, 256, 0),        # 64 tiles: one wave, not split
+                                                (1300, 1008, 5120, 256, 9 * 512)]) # 80 tiles: two rows of the last wave are
 @pytest.mark.parametrize("out", [None, torch.float32])
-def test_split_plan_of_db(M, K, N, gs, out):
+def test_split_plan_of_db(M, K, N, gs, part_rows, out):
+    """The plan, as the rows of fp32 partial sums it asks for (74 CTA pairs), and its dB against the unsplit one and the oracle."""
+    from cute_mma_b200 import _functional as F
+    from cute_mma_b200 import _lib
     rs, dt, act = 16, torch.bfloat16, "sigmoid_gate"
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _lib.lib().prism_workspace_bytes(2, M, N, K, gs, rs, 1, None) == 256 + (part_rows * K * 4 + 255) // 256 * 256
     A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 9)
     dB = cp.backward(dC, A, B, R, gs, rs, activation=act, dB_dtype=out)[2]
+    one = F._backward_db(dC, A, R, gs, rs, 2, out_dtype=out, tile_cfg=[0, -1])
     cp.check_device_status()
     ref = O.prism_backward(dC.float(), A.float(), B.float(), R.float(), gs, rs, act)[2]
     assert dB.dtype == (out or dt) and O.rel_err(dB.float(), ref) < TOL
+    # fp32 sums of at most 2200 products in another order; bf16: each side rounds by up to 2^-8, so that values on two sides
+    # of a rounding boundary end one unit in the last place, 2^-7, apart
+    assert torch.equal(dB, one) if part_rows == 0 else O.rel_err(dB.float(), one.float()) < (1e-5 if out else 2 ** -7 + 1e-5)
 
 
 @pytest.mark.parametrize("G,K,rows", [(1, 64, 1), (3, 192, 33), (5, 1088, 8)])
@@ -338,17 +348,19 @@ def test_tile_width_of_short_forwards(M, N, gs):
     assert O.rel_err(C.float(), O.prism_forward(A.float(), B.float(), R.float(), gs, rs, "silu_gate", bias=bias.float())) < TOL
 
 
+@pytest.mark.parametrize("M", [128, 700])                                        # bf16 silu: stores by TMA; plain ones below 256
 @pytest.mark.parametrize("gs,N", [(16, 48), (32, 64), (96, 192), (256, 512)])   # stores of 16, 32 and 64 rows of dB
 @pytest.mark.parametrize("K", [8, 72, 200, 328])                                 # features that end inside a 64-wide store
-def test_transposed_stores_of_db(gs, N, K):
+@pytest.mark.parametrize("rs,dt,gate", [(8, torch.bfloat16, 1), (16, torch.bfloat16, 1), (16, torch.float16, 2)])
+def test_transposed_stores_of_db(gs, N, K, M, rs, dt, gate):
     """16-bit dB is the rounded fp32 dB, which leaves by plain stores, and touches nothing beside it."""
     from cute_mma_b200 import _functional as F
-    M, rs, dt = 128, 8, torch.bfloat16
+    K -= K % rs if K > rs else K - rs
     A, B, R, dC = _inputs(M, K, N, gs, rs, dt, 23)
     pad = torch.full((N + 2, K), 7.0, dtype=dt, device=DEV)
-    dB = F._backward_db(dC, A, R, gs, rs, 1, dc_scale=0.5, dB_out=pad[1:N + 1])
-    wide = F._backward_db(dC, A, R, gs, rs, 1, dc_scale=0.5, out_dtype=torch.float32)
+    dB = F._backward_db(dC, A, R, gs, rs, gate, dc_scale=0.5, dB_out=pad[1:N + 1], tile_cfg=[0, -1])
+    wide = F._backward_db(dC, A, R, gs, rs, gate, dc_scale=0.5, out_dtype=torch.float32, tile_cfg=[0, -1])
     cp.check_device_status()
     assert torch.equal(dB, wide.to(dt)) and (pad[0] == 7).all() and (pad[N + 1] == 7).all()
-    ref = O.prism_backward(0.5 * dC.float(), A.float(), B.float(), R.float(), gs, rs, "silu_gate")[2]
+    ref = O.prism_backward(0.5 * dC.float(), A.float(), B.float(), R.float(), gs, rs, (None, "silu_gate", "sigmoid_gate")[gate])[2]
     assert O.rel_err(wide, ref) < TOL

@@ -77,3 +77,10 @@ def test_plan_of_db_given_by_hand(plan):
     assert _db(plan, 4096, 4096, 1024, 256, [128, 3, 0, 0, 0, 0, 0, 0]) == (128, 3, 0, 1)
     assert _db(plan, 8192, 5120, 1024, 256, [0, -1, 0, 0, 0, 0, 0, 0]) == (256, 1, 0, 1)
     assert _db(plan, 0, 4096, 1024, 256, [0, 4, 0, 0, 0, 0, 0, 0])[1] == 4
+
+
+@pytest.mark.parametrize("bn,blocks,bf16_silu,tma", [(256, 1, 1, 1), (256, 32, 1, 1), (256, 64, 1, 0), (64, 2, 1, 1), (64, 8, 1, 0),
+                                                     (16, 1, 1, 0), (256, 128, 0, 1), (32, 64, 0, 1), (16, 1, 0, 0),
+                                                     (256, 1 << 24, 1, 0)])
+def test_which_tiles_of_db_leave_by_tma(plan, bn, blocks, bf16_silu, tma):
+    assert plan.plan_db_tma(bn, blocks, bf16_silu) == tma
