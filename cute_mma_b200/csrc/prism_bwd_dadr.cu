@@ -96,23 +96,6 @@ __global__ void __launch_bounds__(256) dadr_reduce_kernel(const DadrReduce p) {
   }
 }
 
-// Groups per part when the tiles alone leave at least half of the SM pairs idle and the groups are split over
-// blockIdx.y (see DadrExtra); G: one part.  A part costs its share of the group steps (about 0.6 us per 64 outputs)
-// plus a pair's start and epilogue; splitting costs the second launch (3 us) and the fp32 sums of dA, written
-// and read once (about 5 TB/s).  Split only for a gain of 2 us or more.
-static int dadr_groups_per_part(int M, int K, int G, int gs, int pairs, int slots) {
-  if (G < 2 || 2 * pairs > slots) return G;
-  const double step = 0.6 * ((gs + 63) / 64);
-  double best_cost = G * step - 2.0;
-  int best = G;
-  for (int parts = 2; parts <= G && pairs * parts <= slots; ++parts) {
-    const int per = (G + parts - 1) / parts;
-    const double cost = per * step + 3.0 + (double)parts * M * K * 8.0 / 5e6;
-    if (cost < best_cost) { best_cost = cost; best = per; }
-  }
-  return best;
-}
-
 // Grid of the dA+dR kernel.  runs: the number of main CTA pairs that share one feature column (each
 // walks every runs-th 256-token tile).  When the main pairs leave SM pairs idle and have enough
 // tiles each, the idle pairs become extra pairs and every main pair leaves its last `steal` tiles

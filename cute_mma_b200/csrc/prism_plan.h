@@ -155,4 +155,24 @@ inline void db_plan(int M, int N, int K, int gs, int sms, const int* cfg, DbPlan
   }
 }
 
+// Groups per part of the dA+dR kernel when the tiles alone (`pairs` CTA pairs of `slots`) leave at least half of the SM pairs idle
+// and the groups are split over blockIdx.y (see DadrExtra); G: one part.  A group takes a pair 1.0 us and 0.2 us per 64
+// outputs in plain mode (1.2 us for 64 outputs, 2.4 for 512, 4.0 for 1024); gates add 0.4 us, an internal bias 1.5, rotations of 32
+// and 64 0.5 and 1.8, which the workspace's size does not know of and the rule leaves out.  A split costs the fp32 sums of dA, written and
+// read once (about 5 TB/s); they are added in the launch that adds dR's.  Split for a gain of 0.5 us or more.
+// Over 300 timed shapes of few tiles (all modes) 0.7 % above the best split in the mean and none slower than unsplit; with
+// 0.6 us per 64 outputs and 5 us against a split, as before, 13 %, up to 2.9 times.
+inline int dadr_groups_per_part(int M, int K, int G, int gs, int pairs, int slots) {
+  if (G < 2 || 2 * pairs > slots) return G;
+  const double step = 1.0 + 0.2 * ((gs + 63) / 64);
+  double best_us = G * step - 0.5;
+  int best = G;
+  for (int parts = 2; parts <= G && pairs * parts <= slots; ++parts) {
+    const int per = (G + parts - 1) / parts;
+    const double us = per * step + (double)parts * M * K * 8.0 / 5e6;
+    if (us < best_us) { best_us = us; best = per; }
+  }
+  return best;
+}
+
 }  // namespace prism

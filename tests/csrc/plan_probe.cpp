@@ -9,3 +9,6 @@ extern "C" void plan_db(int M, int N, int K, int gs, int sms, const int* cfg, in
   out[0] = p.bn; out[1] = p.splits; out[2] = p.tail_rows; out[3] = p.tail_splits;
 }
 extern "C" int plan_db_tma(int bn, int blocks, int bf16_silu) { return prism::db_tma_out(bn, blocks, bf16_silu != 0); }
+extern "C" int plan_dadr_per_part(int M, int K, int G, int gs, int pairs, int slots) {
+  return prism::dadr_groups_per_part(M, K, G, gs, pairs, slots);
+}

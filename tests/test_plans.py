@@ -84,3 +84,23 @@ def test_plan_of_db_given_by_hand(plan):
                                                      (256, 1 << 24, 1, 0)])
 def test_which_tiles_of_db_leave_by_tma(plan, bn, blocks, bf16_silu, tma):
     assert plan.plan_db_tma(bn, blocks, bf16_silu) == tma
+
+
+@pytest.mark.parametrize("M,K,G,gs,pairs,per", [
+    (100, 64, 4, 64, 1, 1),          # four short steps in a row against four pairs side by side
+    (100, 64, 1, 64, 1, 1),          # nothing to split
+    (1024, 768, 3, 256, 24, 3),      # the sums of dA cost what two of three steps save
+    (1024, 4096, 60, 64, 37, 30),    # room for two parts
+    (1024, 4096, 60, 64, 38, 60),    # more than half of the pairs in use
+    (128, 4096, 56, 256, 32, 28)])
+def test_group_parts_of_dadr(plan, M, K, G, gs, pairs, per):
+    assert plan.plan_dadr_per_part(M, K, G, gs, pairs, SMS // 2) == per
+
+
+def test_group_parts_of_dadr_fit_the_pairs(plan):
+    for G in (1, 2, 3, 7, 56, 1000):
+        for pairs in (1, 2, 30, 37, 38, 74, 200):
+            for gs in (16, 256, 1024):
+                per = plan.plan_dadr_per_part(300, 1000, G, gs, pairs, SMS // 2)
+                parts = -(-G // per)
+                assert 1 <= per <= G and (parts == 1 or parts * pairs <= SMS // 2)
