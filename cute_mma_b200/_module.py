@@ -69,7 +69,8 @@ def _kernel_grads(dC, A, B, R, group_size, reconn_sz, activation, bwd_scale, nee
     dC, A, B, R = dC.contiguous(), A.contiguous(), B.contiguous(), R.contiguous()
     gate = F._gate_code(activation or None)
     ib = ib.contiguous() if ib is not None else None
-    seeds = F._check_seeds(seeds, A, B.shape[0] // group_size) if seeds is not None else None   # as the forward took them
+    if seeds is not None and dropout_p > 0.0:   # as the forward took them
+        seeds = F._check_seeds(seeds, A, B.shape[0] // group_size)
     dA, dR, dB, d_ib = F._backward_both(dC, A, B, R, group_size, reconn_sz, gate, bwd_scale, need_dB, ib, seeds, dropout_p)
     if need_dB and not gate:
         dB = torch.zeros_like(B)  # frozen-B contract of the reference's plain mode

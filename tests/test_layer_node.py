@@ -190,3 +190,10 @@ def test_dropout_seeds_reach_the_kernels_as_the_forward_took_them(calls, monkeyp
     for name in ("dadr", "db"):
         given = calls[name]["dropout_seeds"]
         assert given.is_contiguous() and given.device == A.device and torch.equal(given, seeds)
+
+
+def test_seeds_without_dropout_are_not_looked_at(calls):
+    """A probability of 0: the forward ignores the seeds, whatever they are, and so does the backward."""
+    A, B, R, ib = _operands()
+    _layer(A, B, R, ib, seeds=torch.zeros(5), p=0.0).sum().backward()
+    assert calls["dadr"]["dropout_mask"] is None and calls["dadr"]["dropout_p"] == 0.0
