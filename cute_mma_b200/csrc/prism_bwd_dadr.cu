@@ -198,8 +198,8 @@ int launch_bwd_dadr(const DadrArgs& a) {
   const bool drop = a.drop_seeds != nullptr && a.drop_p > 0.f && a.gate != GATE_NONE;
   if (drop && a.E != 16) return fail(PRISM_ERR_UNSUPPORTED, "bwd_dadr: dropout needs reconn_sz 8 or 16");
   x.drop_seeds = a.drop_seeds; x.drop_thr = drop_threshold(a.drop_p); x.drop_mask = a.drop_mask; x.drop_inv_keep = drop ? 1.f / (1.f - a.drop_p) : 1.f;
-  DadrKernel kern = (a.dtype == DT_BF16) ? dadr_kernel_bf16(a.gate, a.E, ib, drop, a.grid.parts > 1)
-                                         : dadr_kernel_f16(a.gate, a.E, ib, drop, a.grid.parts > 1);
+  const bool parts = a.grid.parts > 1 || (dadr_sigmoid16(a.dtype, a.gate, a.E, ib, drop) && !dadr_whole(a.gs));
+  DadrKernel kern = (a.dtype == DT_BF16) ? dadr_kernel_bf16(a.gate, a.E, ib, drop, parts) : dadr_kernel_f16(a.gate, a.E, ib, drop, parts);
   if ((rc = set_max_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd_dadr"))) return rc;
   dim3 grid(2 * (p.n_main + p.n_extra), a.grid.parts, 1);   // the two CTAs of a pair are neighbours
   kern<<<grid, dadr::kThreads, smem_bytes, a.stream>>>(tmA, tmRr, tmRd, tmdC, tmB, p, x);

@@ -243,8 +243,9 @@ __device__ __forceinline__ float* dadr_unit_ib(const DadrParams& p, const DadrEx
 // added in a fixed order, and one thread per column stores (first tile) or adds (later tiles).
 // DROP: hash dropout (see drop_mask32): dH is multiplied by the forward's mask before it is used.
 // PARTS: the groups may be split over blockIdx.y (see DadrExtra).  The instances that can be split run 3 % (fp16) and 1.5 %
-// (plain mode) slower on one part than those that cannot, so both exist; with bf16 gates it is the other way round (fewer
-// spills: 16384 x 4096 -> 14336 4.22 -> 4.00 ms, 8192 x 1024 -> 16384 560 -> 540 us) and there is only the former.
+// (plain mode) slower on one part than those that cannot, so both exist.  With bf16 gates it is the other way round (fewer
+// spills: silu 16384 x 4096 -> 14336 4.22 -> 4.00 ms, 8192 x 1024 -> 8192 with groups of 64 1086 -> 982 us, of 256 295 -> 281; sigmoid
+// of 64 1011 -> 961) and there is only the former, except for sigmoid with groups near 256 (see dadr_whole).
 template <int DT, int GATE, int E, bool IB, bool DROP, bool PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(dadr::kThreads, 1)
 prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmRr,
@@ -806,15 +807,24 @@ prism_bwd_dadr_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 }
 
 using DadrKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, DadrParams, DadrExtra);
-// kernel instance for (gate, E, internal-bias variant, dropout, groups split into parts), one function per data type and
+// kernel instance for (gate, E, internal-bias variant, dropout, whether it has to be or should be the one that can be split), one function per data type and
 // translation unit
 DadrKernel dadr_kernel_f16(int gate, int E, bool ib, bool drop, bool parts);
 DadrKernel dadr_kernel_bf16(int gate, int E, bool ib, bool drop, bool parts);
 
+// bf16 sigmoid without internal bias and dropout, rotations of 8 and 16: the one kind of bf16 gates with both instances
+constexpr bool dadr_sigmoid16(int dt, int gate, int E, bool ib, bool drop) {
+  return dt == DT_BF16 && gate == GATE_SIGMOID && E == 16 && !ib && !drop;
+}
+// ... and when it takes the one that cannot be split, split / whole: 8192 x 1024 -> 8192 with groups of 256 286 / 272 us, of 192 345 /
+// 341, of 160 391 / 411, of 512 222 / 221; 16384 x 2048 -> 4096 with groups of 256 534 / 517.
+inline bool dadr_whole(int gs) { return gs > 192 && gs < 512; }
+
 #define PRISM_DADR_PICK_P(DT_, G_, E_, IB_, DROP_)                                                           \
-  (parts || (DT_ == DT_BF16 && G_ != GATE_NONE)                                                              \
+  (parts || (DT_ == DT_BF16 && G_ != GATE_NONE && !dadr_sigmoid16(DT_, G_, E_, IB_, DROP_))                  \
        ? (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, IB_, DROP_, true>                                     \
-       : (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, IB_, DROP_, (DT_ == DT_BF16 && G_ != GATE_NONE)>)
+       : (DadrKernel)prism_bwd_dadr_kernel<DT_, G_, E_, IB_, DROP_,                                           \
+                                           (DT_ == DT_BF16 && G_ != GATE_NONE && !dadr_sigmoid16(DT_, G_, E_, IB_, DROP_))>)
 #define PRISM_DADR_PICK_IB(DT_, G_, E_, DROP_) \
   (ib ? PRISM_DADR_PICK_P(DT_, G_, E_, true, DROP_) : PRISM_DADR_PICK_P(DT_, G_, E_, false, DROP_))
 #define PRISM_DADR_PICK_G(DT_, E_, DROP_)                                                        \
